@@ -19,25 +19,36 @@
 
 namespace drxg {
 
-constexpr int kBbThreads = 256;
+constexpr int kBbThreads = 128;
 
-/* frames[f][i] ^= prbs[i], i < kbytes; four bytes per thread, grid rows walk
- * the frames */
+/* frames[f][i] ^= prbs[i], i < kbytes: a thread takes the 16-byte blocks at one
+ * place of its rows, aligned in memory, so that full blocks move in one load
+ * and one store whatever the row's own alignment; the sequence's bytes come
+ * from five words, shifted by the row's offset (they stay in L1).  Bound by
+ * the rows' traffic, read and written once: 4096 normal 3/5 frames (40 MB) 19
+ * -> 11 us; four bytes a thread with the sequence loaded byte by byte before. */
 __global__ void __launch_bounds__(kBbThreads) k_bb_descramble(uint8_t* frames, size_t stride, int kbytes,
                                                              int nframes)
 {
+    const int at = 16 * (blockIdx.x * blockDim.x + threadIdx.x);
     for (int f = blockIdx.y; f < nframes; f += gridDim.y) {
-        uint8_t* w = frames + (size_t)f * stride;
-        const bool vec = (((uintptr_t)w) & 3) == 0;
-        for (int i = 4 * (blockIdx.x * blockDim.x + threadIdx.x); i < kbytes; i += 4 * gridDim.x * blockDim.x) {
-            if (vec && i + 4 <= kbytes) {
-                const uint32_t p = (uint32_t)g_bb_prbs[i] | (uint32_t)g_bb_prbs[i + 1] << 8 |
-                                   (uint32_t)g_bb_prbs[i + 2] << 16 | (uint32_t)g_bb_prbs[i + 3] << 24;
-                *(uint32_t*)(w + i) ^= p;
-            } else {
-                for (int k = i; k < i + 4 && k < kbytes; k++)
-                    w[k] ^= g_bb_prbs[k];
-            }
+        uint8_t* row = frames + (size_t)f * stride;
+        const int off = at - (int)((uintptr_t)row & 15); /* of the block, in the row */
+        if (off >= kbytes)
+            continue;
+        if (off >= 0 && off + 16 <= kbytes) {
+            const uint32_t* s = (const uint32_t*)g_bb_prbs + (off >> 2);
+            const uint32_t sh = 8u * (off & 3);
+            uint4 v = *(const uint4*)(row + off);
+            const uint32_t s0 = s[0], s1 = s[1], s2 = s[2], s3 = s[3], s4 = s[4];
+            v.x ^= __funnelshift_r(s0, s1, sh);
+            v.y ^= __funnelshift_r(s1, s2, sh);
+            v.z ^= __funnelshift_r(s2, s3, sh);
+            v.w ^= __funnelshift_r(s3, s4, sh);
+            *(uint4*)(row + off) = v;
+        } else {
+            for (int k = max(off, 0); k < off + 16 && k < kbytes; k++)
+                row[k] ^= g_bb_prbs[k];
         }
     }
 }
@@ -90,7 +101,8 @@ int drx_bb_descramble_device(uint8_t* frames, size_t stride, int kbch_bytes, int
         set_error("drx_bb_descramble_device: bad arguments");
         return -1;
     }
-    const int gx = std::max(1, (kbch_bytes / 4 + kBbThreads - 1) / kBbThreads);
+    /* blocks that rows of any alignment touch: the row's bytes and up to 15 before it */
+    const int gx = ((kbch_bytes + 15) / 16 + 1 + kBbThreads - 1) / kBbThreads;
     const dim3 grid(gx, std::min(nframes, 4096));
     k_bb_descramble<<<grid, kBbThreads, 0, (cudaStream_t)stream>>>(frames, stride, kbch_bytes, nframes);
     return cuda_check(cudaGetLastError(), "descrambler launch") ? 0 : -1;

@@ -36,8 +36,8 @@ def crc8_table():
     return tab
 
 
-def emit(name, vals):
-    lines = ["static __device__ const uint8_t %s[%d] = {" % (name, len(vals))]
+def emit(name, vals, align=""):
+    lines = ["static __device__ %sconst uint8_t %s[%d] = {" % (align, name, len(vals))]
     for i in range(0, len(vals), 16):
         lines.append("    " + ", ".join("0x%02x" % v for v in vals[i:i + 16]) + ",")
     lines.append("};")
@@ -49,7 +49,9 @@ def main(out):
         f.write("/* Generated by dvbrx_b200/tables/gen_bb.py: DVB-S2 BBFRAME scrambling sequence\n"
                 " * (EN 302 307-1 5.2.2) and CRC-8 table (5.1.4). Do not edit. */\n#pragma once\n#include <stdint.h>\n\n")
         f.write("#define DRXG_KBCH_MAX_BYTES %d\n\n" % KBCH_MAX_BYTES)
-        f.write(emit("g_bb_prbs", prbs_bytes(KBCH_MAX_BYTES)) + "\n\n")
+        # read as words from any byte on: aligned, with a word to spare
+        prbs = prbs_bytes(KBCH_MAX_BYTES)
+        f.write(emit("g_bb_prbs", prbs + [0] * (32 - len(prbs) % 16), "__align__(16) ") + "\n\n")
         f.write(emit("g_bb_crc8", crc8_table()) + "\n")
 
 
