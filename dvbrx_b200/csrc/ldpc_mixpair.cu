@@ -28,9 +28,9 @@ namespace drxg {
 /* the shapes behind the switch: (A, B, GDM, LS) of the one-CTA frame-pair
  * kernels that pair_kernel_id picks for the DVB-S2 codes */
 #define DRXG_MIX_SHAPES(X)                                                                               \
-    X(0, 1, 2, 0, 2) X(1, 2, 2, 0, 2) X(2, 3, 3, 0, 2) X(3, 4, 4, 0, 2) X(4, 5, 5, 0, 2) X(5, 8, 8, 0, 2) \
+    X(0, 1, 2, 0, 1) X(1, 2, 2, 0, 1) X(2, 3, 3, 0, 1) X(3, 4, 4, 0, 1) X(4, 5, 5, 0, 1) X(5, 8, 8, 0, 2) \
     X(6, 9, 9, 0, 2) X(7, 12, 12, 0, 2) X(8, 9, 9, 0, 3) X(9, 16, 16, 0, 4) X(10, 20, 20, 0, 3)          \
-    X(11, 25, 25, 0, 6) X(12, 28, 28, 0, 4) X(13, 1, 1, 7, 3) X(14, 1, 1, 14, 3) X(15, 1, 1, 22, 5)
+    X(11, 25, 25, 0, 6) X(12, 28, 28, 0, 4) X(13, 1, 1, 7, 1) X(14, 1, 1, 14, 3) X(15, 1, 1, 22, 5) X(16, 25, 25, 0, 3)
 
 /* One code's frames with its shape: its tables staged in the shape's form,
  * then the streaming loop of the frame-pair kernel. */

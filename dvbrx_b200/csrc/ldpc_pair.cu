@@ -41,8 +41,10 @@ const PairKernel* pair_kernel_part(int part, int* n)
  * id).  Pair kernels by information-link counts (A, B): every pair of the
  * DVB-S2, S2X and T2 codes, plus predicated kernels for the codes whose
  * layers have more than two different counts (degree bounds 7, 11, 14, 22,
- * 32); LS: late slots the kernel carries (two cover most levelled codes;
- * normal 4/5 and 9/10 need four, short 5/6 five, short 8/9 six); residency
+ * 32); LS: half the shared slots the kernel carries (none for the shapes of
+ * the S2X codes alone, which then hold no level code: 18/30 0.339 -> 0.305 us
+ * per frame-iteration; one or two for most levelled codes, three to six from
+ * normal 4/5, short 3/5 and 4/5 up); residency
  * mode 0 (one CTA per SM), and the two-CTA twins (modes 1 and 2) of the
  * kernels that fit 80 registers. */
 static const std::vector<PairKernel>& kernels()

@@ -46,9 +46,8 @@
 namespace drxg {
 
 constexpr int kQCp = 360;
-/* a kernel compiled for LS late slots reads late and writes early only owned
- * slots 1 .. LS of each thread (link slots 2 .. 2 LS + 1); two cover every
- * pair code but short 3/5 and 4/5, which take three */
+/* a kernel compiled for LS reads late and writes early only link slots
+ * 2 .. 2 LS + 1 */
 constexpr int kLateSlotsMax = 6;
 
 /* PRMT in its default mode: a selector nibble with bit 3 set replicates the
@@ -250,7 +249,7 @@ struct PairCheckKey {
     template <bool LEV>
     __device__ __forceinline__ void read_all(const uint16_t* __restrict__ post, uint32_t r0, uint32_t r1)
     {
-        const uint32_t excl = LEV ? (~live | inm) : ~live;
+        const uint32_t excl = LEV ? (~live | inm | outm) : ~live;
         /* slot k read: its value kept in x[k] (minus its old message for a
          * late slot), its key returned */
         auto slot = [&](int k) {
@@ -258,17 +257,17 @@ struct PairCheckKey {
             const uint32_t raw = PO && k < 2 ? (k == 0 ? r0 : r1) : lds16(addr[k]);
             const uint32_t v = sadd(sx2(raw), m);
             uint32_t kv = key(v, k);
-            /* late slots are among K0 .. K1; past them only a non-link (inexact kernels) */
-            const bool maybe_late = LEV && k >= K0 && k <= K1;
-            if (maybe_late || !EXACT || k == 1) {
-                /* excluded: not a link, or late (its sign and key are taken in read_late) */
+            /* shared slots are among K0 .. K1; past them only a non-link (inexact kernels) */
+            const bool maybe_shared = LEV && k >= K0 && k <= K1;
+            if (maybe_shared || !EXACT || k == 1) {
+                /* excluded: not a link, or shared (its sign and key are taken in fold_shared) */
                 const bool ex = (excl >> k) & 1u;
                 kv = ex ? kKeyOff : kv;
                 sg ^= ex ? 0u : v;
             } else {
                 sg ^= v;
             }
-            if (maybe_late)
+            if (maybe_shared)
                 x[k] = ((inm >> k) & 1u) ? m : v;
             else
                 x[k] = v;
@@ -283,6 +282,16 @@ struct PairCheckKey {
         }
         if (S & 1)
             fold(slot(S - 1));
+    }
+
+    /* the smallest magnitude so far */
+    __device__ __forceinline__ uint32_t smallest() const { return (min0 >> 5) & 0x07FF07FFu; }
+
+    /* a shared slot into the minimums and the sign (use: it is one) */
+    __device__ __forceinline__ void fold_shared(int k, bool use)
+    {
+        fold(use ? key(x[k], k) : kKeyOff);
+        sg ^= use ? x[k] : 0u;
     }
 
     /* a thread that holds no check (t >= 360): valid addresses, no links, so
@@ -301,32 +310,13 @@ struct PairCheckKey {
         sg = a0 = a1 = b0 = b1 = nidx = recw = 0;
     }
 
-    /* the late slots (their bits were written by earlier levels) of a check
-     * in the current level (mine); other threads keep their state.  Shared
-     * links come first in every layer (codes.cpp), so late and early slots
-     * are among slots 2 .. KE */
-    template <int KE>
-    __device__ __forceinline__ void read_late(const uint16_t* __restrict__ post, bool mine)
-    {
-        const uint32_t im = mine ? inm : 0u;
-#pragma unroll
-        for (int k = K0; k <= KE; k++) {
-            const bool in = (im >> k) & 1u;
-            const uint32_t v = sadd(sx2(lds16(addr[k])), x[k]);
-            x[k] = in ? v : x[k];
-            sg ^= in ? v : 0u;
-            fold(in ? key(v, k) : kKeyOff);
-        }
-    }
-
     /* the cap at 127 and offset 1, or the learned magnitudes of each lane's
-     * iteration (lpA: the check's class table, learned_lut; lpB unused); the
+     * iteration (lpA: the check's class table, learned_lut); the
      * outgoing candidates +-mn0, +-mn1 with the check's sign parity applied
      * (a0, a1 for a slot whose value is positive, b0 = -a0, b1 = -a1
      * otherwise) and the record's magnitudes.
-     * Only threads with `take` keep the result: the level steps run it on
-     * whole warps */
-    __device__ __forceinline__ void finish(bool take, bool learned, uint32_t lpA, uint32_t lpB)
+     */
+    __device__ __forceinline__ void finish(bool learned, uint32_t lpA)
     {
         const uint32_t c0 = __vmins2((min0 >> 5) & 0x07FF07FFu, 0x007F007Fu);
         const uint32_t c1 = __vmins2((min1 >> 5) & 0x07FF07FFu, 0x007F007Fu);
@@ -338,19 +328,16 @@ struct PairCheckKey {
             m0 = __viaddmax_s16x2(c0, 0xFFFFFFFFu, 0u);
             m1 = __viaddmax_s16x2(c1, 0xFFFFFFFFu, 0u);
         }
-        if (take) {
-            /* both signs of each candidate side by side (the level steps wait on this chain) */
-            const uint32_t sm = lmask(sg), q0 = neg2(m0), q1 = neg2(m1);
-            a0 = sel(sm, q0, m0);
-            a1 = sel(sm, q1, m1);
-            b0 = sel(sm, m0, q0);
-            b1 = sel(sm, m1, q1);
-            nidx = (min0 & 0x001F001Fu) | 0x64006400u; /* FP16 1024 + slot of min0 */
-            /* per lane min0 (6 bits) | min1 << 6, magnitudes capped at 32 (| index << 12 below degree 17) */
-            recw = __vmins2(m0, 0x00200020u) | (__vmins2(m1, 0x00200020u) << 6);
-            if (!WIDE)
-                recw |= (min0 & 0x000F000Fu) << 12;
-        }
+        const uint32_t sm = lmask(sg), q0 = neg2(m0), q1 = neg2(m1);
+        a0 = sel(sm, q0, m0);
+        a1 = sel(sm, q1, m1);
+        b0 = sel(sm, m0, q0);
+        b1 = sel(sm, m1, q1);
+        nidx = (min0 & 0x001F001Fu) | 0x64006400u; /* FP16 1024 + slot of min0 */
+        /* per lane min0 (6 bits) | min1 << 6, magnitudes capped at 32 (| index << 12 below degree 17) */
+        recw = __vmins2(m0, 0x00200020u) | (__vmins2(m1, 0x00200020u) << 6);
+        if (!WIDE)
+            recw |= (min0 & 0x000F000Fu) << 12;
     }
 
     /* new posterior of slot k (two bytes) and the lane mask of its value's sign */
@@ -361,21 +348,6 @@ struct PairCheckKey {
         const uint32_t eq = heq(nidx, 0x64006400u + (uint32_t)k * 0x00010001u);
         const uint32_t o = sel(xm, sel(eq, b1, b0), sel(eq, a1, a0));
         return pk2(sadd(v, o));
-    }
-
-    /* posteriors that later levels of the layer read (checks of the current
-     * level only) */
-    template <int KE>
-    __device__ __forceinline__ void write_early(uint16_t* __restrict__ post, bool mine) const
-    {
-        const uint32_t om = mine ? outm : 0u;
-#pragma unroll
-        for (int k = K0; k <= KE; k++) {
-            uint32_t xm;
-            const uint32_t nv = update(k, xm);
-            if ((om >> k) & 1u)
-                sts16(addr[k], nv);
-        }
     }
 
     /* every other posterior (predicated stores) and the node's compressed
@@ -506,18 +478,19 @@ struct PairCheckMin {
     template <bool LEV>
     __device__ __forceinline__ void read_all(const uint16_t* __restrict__ post, uint32_t r0, uint32_t r1)
     {
-        const uint32_t excl = LEV ? (~live | inm) : ~live;
+        const uint32_t shared = inm | outm;
         uint32_t f[S];
 #pragma unroll
         for (int k = 0; k < S; k++) {
             const uint32_t m = unmsg(k);
             const uint32_t raw = PO && k < 2 ? (k == 0 ? r0 : r1) : lds16(addr[k]);
             uint32_t v = sadd(sx2(raw), m);
-            if (LEV || !EXACT || k == 1)
-                v = ((excl >> k) & 1u) ? 0x00FF00FFu : v;
-            f[k] = v;
-            /* a late slot keeps minus its old message for read_late */
-            x[k] = LEV && ((inm >> k) & 1u) ? m : v;
+            if (!EXACT || k == 1) /* a slot that can be absent: above every minimum */
+                v = ((live >> k) & 1u) ? v : 0x00FF00FFu;
+            const bool maybe_shared = LEV && k >= K0 && k <= K1;
+            f[k] = maybe_shared && ((shared >> k) & 1u) ? 0x00FF00FFu : v;
+            /* a late slot keeps minus its old message for its level */
+            x[k] = maybe_shared && ((inm >> k) & 1u) ? m : v;
         }
 #pragma unroll
         for (int k = 0; k + 1 < S; k += 2) {
@@ -530,6 +503,12 @@ struct PairCheckMin {
         if (S & 1)
             fold(f[S - 1]);
     }
+
+    /* the smallest magnitude so far */
+    __device__ __forceinline__ uint32_t smallest() const { return min0; }
+
+    /* a shared slot into the minimums and the sign (use: it is one) */
+    __device__ __forceinline__ void fold_shared(int k, bool use) { fold(use ? x[k] : 0x00FF00FFu); }
 
     /* a thread that holds no check (t >= 360): valid addresses, no links, so
      * that it can run the warp-uniform level steps of its warp */
@@ -547,28 +526,10 @@ struct PairCheckMin {
         sg = mn0 = mn1 = m0p1 = nmn0 = nmn1 = 0;
     }
 
-    /* the late slots (their bits were written by earlier levels) of a check
-     * in the current level (mine); other threads keep their state.  Shared
-     * links come first in every layer (codes.cpp), so late and early slots
-     * are among slots 2 .. KE */
-    template <int KE>
-    __device__ __forceinline__ void read_late(const uint16_t* __restrict__ post, bool mine)
-    {
-        const uint32_t im = mine ? inm : 0u;
-#pragma unroll
-        for (int k = K0; k <= KE; k++) {
-            const bool in = (im >> k) & 1u;
-            const uint32_t v = sadd(sx2(lds16(addr[k])), x[k]);
-            x[k] = in ? v : x[k];
-            fold(in ? v : 0x00FF00FFu);
-        }
-    }
-
     /* the cap at 127 and offset 1, or the learned magnitudes of each lane's
-     * iteration (lpA: the check's class table, learned_lut; lpB unused).
-     * Only threads with `take` keep the result: the level steps run it on
-     * whole warps */
-    __device__ __forceinline__ void finish(bool take, bool learned, uint32_t lpA, uint32_t lpB)
+     * iteration (lpA: the check's class table, learned_lut).
+     */
+    __device__ __forceinline__ void finish(bool learned, uint32_t lpA)
     {
         const uint32_t c1 = min1, c0 = min0;
         uint32_t m0, m1;
@@ -579,13 +540,11 @@ struct PairCheckMin {
             m0 = __viaddmax_s16x2(__vmins2(c0, 0x007F007Fu), 0xFFFFFFFFu, 0u);
             m1 = __viaddmax_s16x2(__vmins2(c1, 0x007F007Fu), 0xFFFFFFFFu, 0u);
         }
-        if (take) {
-            mn0 = m0;
-            mn1 = m1;
-            m0p1 = __vadd2(c0, 0x00010001u);
-            nmn0 = neg2(m0);
-            nmn1 = neg2(m1);
-        }
+        mn0 = m0;
+        mn1 = m1;
+        m0p1 = __vadd2(c0, 0x00010001u);
+        nmn0 = neg2(m0);
+        nmn1 = neg2(m1);
     }
 
     /* new posterior of slot k (two bytes), and its masks: lanes where
@@ -599,21 +558,6 @@ struct PairCheckMin {
         neg = lmask(sg ^ v);
         const uint32_t o = sel(neg, sel(above, nmn0, nmn1), sel(above, mn0, mn1));
         return pk2(sadd(v, o));
-    }
-
-    /* posteriors that later levels of the layer read (checks of the current
-     * level only) */
-    template <int KE>
-    __device__ __forceinline__ void write_early(uint16_t* __restrict__ post, bool mine) const
-    {
-        const uint32_t om = mine ? outm : 0u;
-#pragma unroll
-        for (int k = K0; k <= KE; k++) {
-            uint32_t above, neg;
-            const uint32_t nv = update(k, above, neg);
-            if ((om >> k) & 1u)
-                sts16(addr[k], nv);
-        }
     }
 
     /* every other posterior (predicated stores) and the node's compressed
@@ -653,7 +597,7 @@ struct PairCheckMin {
  * shared links, and check degrees 22 and above), the min form elsewhere. */
 __host__ __device__ constexpr bool pair_key_form(int a, int b, int gdm, int ls)
 {
-    return gdm == 0 && ((a == b && (a == 5 || a == 9) && ls == 2) || a >= 20);
+    return gdm == 0 && ((a == b && (a == 5 || a == 9) && ls <= 2) || a >= 20);
 }
 
 template <int DM, bool EXACT, int LS, bool WIDE, bool PO, bool KEYS>
@@ -849,14 +793,103 @@ __device__ int syndrome_pair(const DevCode& c, const PairFrame& fr, volatile int
 }
 
 /*
+ * The step of a wavefront level, on whole warps: the checks of the level
+ * (mine) read their late slots (late: any level but the first) and write the
+ * posteriors that later levels read (early slots).  A level waits for the one
+ * before it, so the step is kept to the chain from a late slot's posterior to
+ * an early slot's: the message to a shared slot has the magnitude of the
+ * smallest other link, min(inner, the other shared slots), where `inner`, the
+ * outgoing magnitude of the links no other check of the layer shares, is
+ * known before the first level, and the sign of the others' signs.  The
+ * node's minimums take the shared slots after the last level (fold_shared).
+ * Shared links come first in every layer (codes.cpp), so they are among slots
+ * 2 .. KE: two for KE = 3, three or four for KE = 5.
+ * lp: the check's learned class table (learned kernels; inner is then the
+ * capped minimum itself).
+ *
+ * Bound by that chain's latency, 3 to 4 warps a level between CTA barriers: it
+ * took the node's whole finish (minimums, both candidates, the index) and every
+ * shared slot's update before.  With two, four, six and more slots compiled
+ * apart, us of the GPU per frame-iteration: normal 3/5 0.400 -> 0.376, 1/3
+ * 0.426 -> 0.378, 5/6 0.407 -> 0.340, 8/9 0.360 -> 0.264, short 1/2 0.095 ->
+ * 0.086, 3/5 0.181 -> 0.143, 5/6 0.182 -> 0.157.
+ */
+template <int KE, class Ck>
+__device__ __forceinline__ void read_late(Ck& ck, bool mine)
+{
+    const uint32_t im = mine ? ck.inm : 0u;
+#pragma unroll
+    for (int k = Ck::K0; k <= KE; k++) {
+        const uint32_t v = sadd(sx2(lds16(ck.addr[k])), ck.x[k]);
+        ck.x[k] = (im >> k) & 1u ? v : ck.x[k];
+    }
+}
+
+template <int KE, bool LEARNED, class Ck>
+__device__ __forceinline__ void level_step(Ck& ck, uint32_t inner, bool mine, bool late, uint32_t lp)
+{
+    constexpr uint32_t NONE = 0x00FF00FFu; /* above every magnitude */
+    const uint32_t im = mine ? ck.inm : 0u, om = mine ? ck.outm : 0u, sh = ck.inm | ck.outm;
+    /* max(|x| - 1, 0), by -x - 1 = ~x; |x| in learned kernels */
+    auto mag = [](uint32_t v) { return LEARNED ? abs2(v) : __viaddmax_s16x2_relu(v, 0xFFFFFFFFu, ~v); };
+    auto read = [&](int k) {
+        if (late) {
+            const uint32_t v = sadd(sx2(lds16(ck.addr[k])), ck.x[k]);
+            ck.x[k] = (im >> k) & 1u ? v : ck.x[k];
+        }
+        return mag(ck.x[k]);
+    };
+    /* slot k, the smallest magnitude and the sign of the other shared slots */
+    auto write = [&](int k, uint32_t others, uint32_t sign) {
+        const uint32_t v = ck.x[k], r = __vmins2(inner, others);
+        const uint32_t m = LEARNED ? learned_lut(r, lp) : r;
+        /* both signs side by side: v - m = (v + 1) + ~m */
+        const uint32_t up = sadd(v, m), down = sadd(__vadd2(v, 0x00010001u), ~m);
+        const uint32_t nv = pk2(sel(lmask(ck.sg ^ sign), down, up));
+        if ((om >> k) & 1u)
+            sts16(ck.addr[k], nv);
+    };
+    if constexpr (KE == 3) {
+        const uint32_t a = read(2), b = read(3);
+        write(2, b, ck.x[3]);
+        write(3, a, ck.x[2]);
+    } else if constexpr (KE == 5) { /* three or four */
+        const bool four = (sh >> 5) & 1u;
+        const uint32_t a = read(2), b = read(3), c = read(4), r5 = read(5);
+        const uint32_t d = four ? r5 : NONE;
+        const uint32_t ab = __vmins2(a, b), cd = __vmins2(c, d);
+        const uint32_t sab = ck.x[2] ^ ck.x[3], s5 = four ? ck.x[5] : 0u, scd = ck.x[4] ^ s5;
+        write(2, __vmins2(b, cd), ck.x[3] ^ scd);
+        write(3, __vmins2(a, cd), ck.x[2] ^ scd);
+        write(4, __vmins2(ab, d), sab ^ s5);
+        write(5, __vmins2(ab, c), sab ^ ck.x[4]);
+    } else {
+        /* the two smallest: a slot that holds the smallest takes the second */
+        uint32_t m0 = NONE, m1 = NONE, sign = 0;
+#pragma unroll
+        for (int k = Ck::K0; k <= KE; k++) {
+            const bool is = (sh >> k) & 1u;
+            const uint32_t r = read(k), g = is ? r : NONE;
+            m1 = __vmins2(m1, __vmaxs2(m0, g));
+            m0 = __vmins2(m0, g);
+            sign ^= is ? ck.x[k] : 0u;
+        }
+#pragma unroll
+        for (int k = Ck::K0; k <= KE; k++)
+            write(k, sel(heq(mag(ck.x[k]), m0), m1, m0), sign ^ ck.x[k]);
+    }
+}
+
+/*
  * Layer i of the phased schedule.  Every check reads its links that no
- * earlier check of the layer writes (a full-occupancy pass); then, level by
- * level, the checks of the level read their remaining links (written by
- * earlier levels), finish their minimums and write only the posteriors that
- * later checks of the layer read; a last full pass writes every other
- * posterior and the messages.  The reference's in-order semantics only
- * constrain the bits two checks of a layer share, so the wavefront levels
- * carry just those links.  Unlevelled layers take one pass.
+ * other check of the layer shares, or that no earlier check writes (a
+ * full-occupancy pass); then, level by level, the checks of the level read
+ * their late links and write the posteriors that later checks of the layer
+ * read (level_step); a last full pass folds the shared links into the
+ * minimums and writes every other posterior and the messages.  The
+ * reference's in-order semantics only constrain the bits two checks of a
+ * layer share, so the wavefront levels carry just those links.  Unlevelled
+ * layers take one pass.
  */
 template <int DM, bool EXACT, int LS, bool WIDE, bool LEARNED, bool PO, bool KEYS>
 __device__ __forceinline__ void layer_pair(const PairFrame& fr, const DevCode& c, int i, int cnt, int nlev,
@@ -868,62 +901,64 @@ __device__ __forceinline__ void layer_pair(const PairFrame& fr, const DevCode& c
     const bool active = t < kQCp;
     const int j = t;
     /* the check's learned class table (an index into s_learn_lut) */
-    auto lwords = [&](uint32_t& a, uint32_t& b) {
-        a = b = 0;
-        if (LEARNED)
-            a = 128u * (uint32_t)s_learn_cls[(EXACT ? DM : cnt + 2) - ((i | j) == 0)];
+    auto lclass = [&]() {
+        return LEARNED ? 128u * (uint32_t)s_learn_cls[(EXACT ? DM : cnt + 2) - ((i | j) == 0)] : 0u;
     };
     using Ck = PairCheck<DM, EXACT, LS, WIDE, PO, KEYS>;
     Ck ck;
     if (active) {
         ck.setup(fr.ent + fr.eoff[i], cnt, c.K, c.q, i, j, rec, fresh, meta,
                  (uint32_t)__cvta_generic_to_shared(fr.post));
-        if (nlev > 1)
+        if (LS > 0 && nlev > 1)
             ck.template read_all<true>(fr.post, r0, r1);
         else
             ck.template read_all<false>(fr.post, r0, r1);
     } else {
         ck.idle((uint32_t)__cvta_generic_to_shared(fr.post));
     }
-    if (nlev > 1) {
+    uint32_t lp = 0;
+    if (active)
+        lp = lclass();
+    if (LS > 0 && nlev > 1) {
         /* a level step runs on every warp that holds a check of the level,
          * with all its lanes; the other checks keep their state.  KE: the
          * last slot that can be late or early in this warp (most
          * layers share one pair of links: link slots 2 and 3 only) */
         const int lev = active ? (int)(meta & 0xFF) : -1;
-        uint32_t wa, wb; /* the check's learned words, read once for all its level steps */
-        lwords(wa, wb);
+        const uint32_t cap = __vmins2(ck.smallest(), 0x007F007Fu);
+        const uint32_t inner = LEARNED ? cap : __viaddmax_s16x2(cap, 0xFFFFFFFFu, 0u);
         auto steps = [&](auto ke) {
             constexpr int KE = decltype(ke)::value;
-            /* every level ends with a CTA barrier, the last one too: without
-             * it the write pass of the other warps takes issue slots from the
-             * last level's chain and the layer runs longer (measured), and
-             * skipping the last level's early writes (it has none to store)
-             * measured slower as well */
-            for (int l = 0; l < nlev; l++) {
+            for (int l = 0; l < nlev - 1; l++) {
                 const bool mine = lev == l;
-                if (__any_sync(0xFFFFFFFFu, mine)) {
-                    if (l > 0)
-                        ck.template read_late<KE>(fr.post, mine);
-                    ck.finish(mine, LEARNED, wa, wb);
-                    ck.template write_early<KE>(fr.post, mine);
-                }
+                if (__any_sync(0xFFFFFFFFu, mine))
+                    level_step<KE, LEARNED>(ck, inner, mine, l > 0, lp);
                 __syncthreads();
             }
+            /* the last level writes nothing early and nothing waits for it */
+            if (__any_sync(0xFFFFFFFFu, lev == nlev - 1))
+                read_late<KE>(ck, lev == nlev - 1);
+            const uint32_t sh = ck.inm | ck.outm;
+#pragma unroll
+            for (int k = Ck::K0; k <= KE; k++)
+                ck.fold_shared(k, KE == 3 || ((sh >> k) & 1u));
         };
-        constexpr int KS = Ck::K1 > 3 ? 3 : Ck::K1;
+        constexpr int KS = Ck::K1 > 3 ? 3 : Ck::K1, KM = Ck::K1 > 5 ? 5 : Ck::K1,
+                      KL = Ck::K1 > 7 ? 7 : Ck::K1;
         const uint32_t lm = __reduce_or_sync(0xFFFFFFFFu, ck.inm | ck.outm);
-        if (KS < Ck::K1 && (lm >> (KS + 1)) != 0)
-            steps(std::integral_constant<int, Ck::K1>());
-        else
+        if (KS == Ck::K1 || (lm >> (KS + 1)) == 0)
             steps(std::integral_constant<int, KS>());
-    } else if (active) {
-        uint32_t wa, wb;
-        lwords(wa, wb);
-        ck.finish(true, LEARNED, wa, wb);
+        else if (KM == Ck::K1 || (lm >> (KM + 1)) == 0)
+            steps(std::integral_constant<int, KM>());
+        else if (KL == Ck::K1 || (lm >> (KL + 1)) == 0)
+            steps(std::integral_constant<int, KL>());
+        else
+            steps(std::integral_constant<int, Ck::K1>());
     }
-    if (active)
+    if (active) {
+        ck.finish(LEARNED, lp);
         ck.write_rest(fr.post, msg + kQCp * i + j, o0, o1);
+    }
     __syncthreads();
 }
 
@@ -1235,8 +1270,7 @@ __global__ void __launch_bounds__(384, PM ? 2 : 1) k_decode_pair(DecodeParams p)
 /* Pair kernels by information-link counts (A, B): every pair of the DVB-S2,
  * S2X and T2 codes, plus predicated kernels for the codes whose layers have
  * more than two different counts (degree bounds 7, 11, 14, 22, 32).  LS:
- * late slots the kernel carries (two cover most levelled codes; normal 4/5
- * and 9/10 need four, short 5/6 five, short 8/9 six). */
+ * half the shared slots the kernel carries. */
 struct PairKernel {
     int a, b, gdm, ls, pm, threads;
     const void* fn;

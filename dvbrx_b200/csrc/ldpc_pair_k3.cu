@@ -7,15 +7,15 @@
 namespace drxg {
 
 static const PairKernel kPart[] = {
-    DRXG_PAIR_KERNEL(5, 5, 0, 2, 2),
-    DRXG_PAIR_KERNEL(5, 6, 0, 2, 1),
-    DRXG_PAIR_KERNEL(5, 6, 0, 2, 2),
-    DRXG_PAIR_KERNEL(6, 7, 0, 2, 1),
-    DRXG_PAIR_KERNEL(6, 7, 0, 2, 2),
-    DRXG_PAIR_KERNEL(7, 7, 0, 2, 1),
-    DRXG_PAIR_KERNEL(7, 7, 0, 2, 2),
-    DRXG_PAIR_KERNEL(7, 8, 0, 2, 1),
-    DRXG_PAIR_KERNEL(7, 8, 0, 2, 2),
+    DRXG_PAIR_KERNEL(5, 5, 0, 1, 2),
+    DRXG_PAIR_KERNEL(5, 6, 0, 0, 1),
+    DRXG_PAIR_KERNEL(5, 6, 0, 0, 2),
+    DRXG_PAIR_KERNEL(6, 7, 0, 0, 1),
+    DRXG_PAIR_KERNEL(6, 7, 0, 0, 2),
+    DRXG_PAIR_KERNEL(7, 7, 0, 0, 1),
+    DRXG_PAIR_KERNEL(7, 7, 0, 0, 2),
+    DRXG_PAIR_KERNEL(7, 8, 0, 0, 1),
+    DRXG_PAIR_KERNEL(7, 8, 0, 0, 2),
     DRXG_PAIR_KERNEL(8, 8, 0, 2, 1),
     DRXG_PAIR_KERNEL(8, 8, 0, 2, 2),
 };

@@ -7,16 +7,16 @@
 namespace drxg {
 
 static const PairKernel kPart[] = {
-    DRXG_PAIR_KERNEL(8, 9, 0, 2, 1),
-    DRXG_PAIR_KERNEL(8, 9, 0, 2, 2),
+    DRXG_PAIR_KERNEL(8, 9, 0, 0, 1),
+    DRXG_PAIR_KERNEL(8, 9, 0, 0, 2),
     DRXG_PAIR_KERNEL(9, 9, 0, 2, 1),
     DRXG_PAIR_KERNEL(9, 9, 0, 2, 2),
-    DRXG_PAIR_KERNEL(9, 10, 0, 2, 1),
-    DRXG_PAIR_KERNEL(9, 10, 0, 2, 2),
-    DRXG_PAIR_KERNEL(11, 11, 0, 2, 1),
-    DRXG_PAIR_KERNEL(11, 11, 0, 2, 2),
-    DRXG_PAIR_KERNEL(11, 12, 0, 2, 1),
-    DRXG_PAIR_KERNEL(11, 12, 0, 2, 2),
+    DRXG_PAIR_KERNEL(9, 10, 0, 0, 1),
+    DRXG_PAIR_KERNEL(9, 10, 0, 0, 2),
+    DRXG_PAIR_KERNEL(11, 11, 0, 0, 1),
+    DRXG_PAIR_KERNEL(11, 11, 0, 0, 2),
+    DRXG_PAIR_KERNEL(11, 12, 0, 0, 1),
+    DRXG_PAIR_KERNEL(11, 12, 0, 0, 2),
     DRXG_PAIR_KERNEL(12, 12, 0, 2, 1),
 };
 

@@ -10,8 +10,8 @@ static const PairKernel kPart[] = {
     DRXG_PAIR_KERNEL(12, 12, 0, 2, 2),
     DRXG_PAIR_KERNEL(9, 9, 0, 3, 1),
     DRXG_PAIR_KERNEL(9, 9, 0, 3, 2),
-    DRXG_PAIR_KERNEL(1, 1, 7, 3, 1),
-    DRXG_PAIR_KERNEL(1, 1, 7, 3, 2),
+    DRXG_PAIR_KERNEL(1, 1, 7, 1, 1),
+    DRXG_PAIR_KERNEL(1, 1, 7, 1, 2),
     DRXG_PAIR_KERNEL(1, 1, 11, 3, 1),
     DRXG_PAIR_KERNEL(1, 1, 11, 3, 2),
     DRXG_PAIR_KERNEL(1, 1, 14, 3, 1),
