@@ -945,9 +945,10 @@ int drx_channel_generate(drx_ldpc* d, const char* constellation, const char* con
         e += (double)row->points[2 * i] * row->points[2 * i] + (double)row->points[2 * i + 1] * row->points[2 * i + 1];
     const float g = (float)(1.0 / sqrt(e / np)); /* unit average energy, as demap.c:183-187 */
     for (int i = 0; i < np; i++) {
-        p.re[i] = row->points[2 * i] * g;
-        p.im[i] = row->points[2 * i + 1] * g;
-        p.e[i] = p.re[i] * p.re[i] + p.im[i] * p.im[i];
+        const float re = row->points[2 * i] * g, im = row->points[2 * i + 1] * g;
+        p.ar[i] = -2.0f * re;
+        p.ai[i] = -2.0f * im;
+        p.e[i] = re * re + im * im;
     }
     for (int b = 0; b < 8; b++)
         p.order[b] = row->order[b] < 0 ? 0 : row->order[b];
@@ -957,7 +958,8 @@ int drx_channel_generate(drx_ldpc* d, const char* constellation, const char* con
     p.llr_f16_stride = llr_f16_stride;
     p.info = info;
     p.info_stride = info_stride;
-    return cuda_ok(launch_channel(p, nframes, d->code.N, stream ? (cudaStream_t)stream : d->stream),
+    return cuda_ok(launch_channel(p, nframes, d->code.N, d->code.K, d->code.q, d->sms,
+                                  stream ? (cudaStream_t)stream : d->stream),
                    "channel launch") ? 0 : -1;
 }
 

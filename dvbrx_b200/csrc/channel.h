@@ -18,7 +18,8 @@ struct ChannelParams {
     int bits;      /* bits per symbol */
     int qpsk;      /* closed-form QPSK, bits 2j and 2j+1 (no interleaver) */
     int order[8];  /* bit-interleaver column of label bit b */
-    float re[256], im[256], e[256]; /* unit-energy points by label, |p|^2 */
+    int parts;     /* CTAs per frame (set by launch_channel) */
+    float ar[256], ai[256], e[256]; /* unit-energy points by label: -2 re, -2 im, |p|^2 */
     int8_t* llr;   /* nframes rows, or null */
     size_t llr_stride;
     __half* llr_f16; /* nframes rows of unquantised LLRs, or null */
@@ -27,6 +28,6 @@ struct ChannelParams {
     size_t info_stride;
 };
 
-cudaError_t launch_channel(const ChannelParams& p, int nframes, int N, cudaStream_t s);
+cudaError_t launch_channel(const ChannelParams& p, int nframes, int N, int K, int q, int sms, cudaStream_t s);
 
 }  // namespace drxg
