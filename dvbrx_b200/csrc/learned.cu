@@ -18,23 +18,29 @@
  * rounding).  The loss is the binary cross-entropy of the information bits
  * after every iteration: sum_t sum_v softplus(-(1 - 2 b_v) P_v / 2).
  *
- * Forward (k_learned_fwd): one CTA per frame, state in global memory
- * (posteriors N floats, messages slots x DS floats, edge-major), and, when
- * training, a checkpoint of (P, m) at the start of every iteration.
+ * One CTA per frame, thread j holding check j of every layer; posteriors in
+ * global memory, a check's messages as one 16-byte record (the two magnitudes,
+ * the outgoing signs, the link that holds the minimum), exact in fp32.  Degrees
+ * are compiled in classes, so a check's links stay in registers.  A layer's
+ * checks load every link no earlier check of the layer writes at once; then
+ * the wavefront levels in turn load the links that earlier ones wrote.
  *
- * Backward (k_learned_bwd): for t = T-1 .. 0 it restores the iteration-t
- * checkpoint, re-runs iteration t saving every extrinsic input x (one float
- * per link), adds the iteration's loss gradient, then walks the steps in
- * reverse: the gradient of a check node's outputs goes to its inputs through
- * the straight path (P' = x + m'), the scale and offset, and the minimum
- * (the argmin link receives d mag / d mu; the sign is piecewise constant);
- * saturated clamps pass no gradient.  Memory is bounded by one checkpoint
- * per iteration instead of every intermediate.
+ * Forward (k_learned_fwd): when training, every iteration leaves its extrinsic
+ * inputs (one float per link) and its information posteriors.
+ *
+ * Backward (k_learned_bwd): for t = T-1 .. 0 it adds the iteration's loss
+ * gradient, from the saved posteriors, then walks the layers and levels in
+ * reverse from the saved extrinsic inputs, which give back the check node: the
+ * gradient of a check node's outputs goes to its inputs through the straight
+ * path (P' = x + m'), the scale and offset, and the minimum (the argmin link
+ * receives d mag / d mu; the sign is piecewise constant); saturated clamps
+ * pass no gradient.
  */
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "codes.h"
 #include "learned.h"
 
 namespace drxg {
@@ -46,186 +52,77 @@ __device__ __forceinline__ float clampf(float v, float lo, float hi) { return fm
 __device__ __forceinline__ float softplus(float u) { return fmaxf(u, 0.0f) + log1pf(expf(-fabsf(u))); }
 __device__ __forceinline__ float sigmoid(float u) { return 1.0f / (1.0f + expf(-u)); }
 
-struct LFrame {
-    float* P;  /* N */
-    float* M;  /* DS * R, edge-major: link c of slot s at c * R + s */
-    float* X;  /* same layout, extrinsic inputs of the current iteration */
-    float* gP; /* N */
-    float* gM; /* DS * R */
+/* The code's link tables, staged in shared memory. */
+struct LTables {
+    const int2* ent;
+    const uint16_t* eoff;
+    const uint8_t* nlev;
 };
 
-__device__ __forceinline__ LFrame frame_state(const LearnedParams& p, int f)
+__device__ LTables stage_tables(const DevCode& c, char* smem)
 {
-    const DevCode& c = *p.code;
-    const size_t E = (size_t)p.DS * c.R;
-    LFrame s;
-    s.P = p.P + (size_t)f * c.N;
-    s.M = p.M + (size_t)f * E;
-    s.X = p.X ? p.X + (size_t)f * E : nullptr;
-    s.gP = p.gP ? p.gP + (size_t)f * c.N : nullptr;
-    s.gM = p.gM ? p.gM + (size_t)f * E : nullptr;
-    return s;
+    int2* ent = (int2*)smem;
+    uint16_t* eoff = (uint16_t*)(ent + c.nent);
+    uint8_t* nlev = (uint8_t*)(eoff + c.q + 1);
+    for (int k = threadIdx.x; k < c.nent; k += blockDim.x)
+        ent[k] = c.ent[k];
+    for (int k = threadIdx.x; k <= c.q; k += blockDim.x)
+        eoff[k] = c.eoff[k];
+    for (int k = threadIdx.x; k < c.q; k += blockDim.x)
+        nlev[k] = c.nlev[k];
+    return LTables{ ent, eoff, nlev };
 }
 
-/* Links of check (i, j) at step position pos: slot 0 = parity, slot 1 =
- * previous parity (absent for (0, 0)), 2.. = information bits. */
-__device__ __forceinline__ int link_var(const DevCode& c, int i, int j, int slot)
+/* Links of check (i, j): slot 0 = parity, slot 1 = previous parity (absent
+ * for (0, 0)), 2.. = information bits (ent: the layer's entries). */
+__device__ __forceinline__ int link_var(const DevCode& c, const int2* ent, int i, int j, int slot)
 {
     if (slot == 0)
         return c.K + kQCl * i + j;
     if (slot == 1)
         return i ? c.K + kQCl * (i - 1) + j : c.K + kQCl * (c.q - 1) + j - 1;
-    const int2 e = c.ent[c.eoff[i] + slot - 2];
+    const int2 e = ent[slot - 2];
     return e.x + j + (j < e.y ? kQCl : 0);
 }
 
-/* Forward of one check; X saved when non-null. */
-__device__ void check_fwd(const DevCode& c, const LFrame& s, int i, int j, int slotpos, float beta, float alpha,
-                          bool first)
-{
-    const int cnt = c.eoff[i + 1] - c.eoff[i];
-    const int D = cnt + 2;
-    const bool has_pp = (i | j) != 0;
-    float x[kLearnedMaxDeg];
-    int var[kLearnedMaxDeg];
-    float min0 = 1e30f, min1 = 1e30f;
-    int a0 = -1;
-    int neg = 0;
-    for (int k = 0; k < D; k++) {
-        if (k == 1 && !has_pp)
-            continue;
-        var[k] = link_var(c, i, j, k);
-        const size_t e = (size_t)k * c.R + slotpos;
-        const float raw = s.P[var[k]] - (first ? 0.0f : s.M[e]);
-        if (s.X)
-            s.X[e] = raw;
-        const float xv = clampf(raw, -128.0f, 127.0f);
-        x[k] = xv;
-        const float a = fabsf(xv);
-        if (a < min0) {
-            min1 = min0;
-            min0 = a;
-            a0 = k;
-        } else if (a < min1) {
-            min1 = a;
-        }
-        neg ^= xv < 0.0f;
-    }
-    for (int k = 0; k < D; k++) {
-        if (k == 1 && !has_pp)
-            continue;
-        const float mu = fminf(k == a0 ? min1 : min0, 127.0f);
-        const float mag = fmaxf(beta * mu - alpha, 0.0f);
-        const bool sneg = neg ^ (x[k] < 0.0f);
-        const float m = sneg ? -mag : mag;
-        s.P[var[k]] = clampf(x[k] + m, -128.0f, 127.0f);
-        s.M[(size_t)k * c.R + slotpos] = clampf(m, -32.0f, 31.0f);
-    }
-}
-
-/* Backward of one check from its saved extrinsic inputs: reads the
- * gradients of its outputs (gP at its links, gM of its messages), writes
- * those of its inputs in their place, accumulates the parameter gradients. */
-__device__ void check_bwd(const DevCode& c, const LFrame& s, int i, int j, int slotpos, float beta, float alpha,
-                          bool first, float& dbeta, float& dalpha)
-{
-    const int cnt = c.eoff[i + 1] - c.eoff[i];
-    const int D = cnt + 2;
-    const bool has_pp = (i | j) != 0;
-    float raw[kLearnedMaxDeg], x[kLearnedMaxDeg], gx[kLearnedMaxDeg];
-    int var[kLearnedMaxDeg];
+/* The smallest two magnitudes among a check's inputs, the links that hold
+ * them (the first of equal ones), those links' signs and all signs' parity. */
+struct Node {
     float min0 = 1e30f, min1 = 1e30f;
     int a0 = -1, a1 = -1;
-    int neg = 0;
-    for (int k = 0; k < D; k++) {
-        if (k == 1 && !has_pp)
-            continue;
-        var[k] = link_var(c, i, j, k);
-        raw[k] = s.X[(size_t)k * c.R + slotpos];
-        const float xv = clampf(raw[k], -128.0f, 127.0f);
-        x[k] = xv;
-        gx[k] = 0.0f;
+    bool n0 = false, n1 = false, neg = false;
+    __device__ __forceinline__ void add(float xv, int k)
+    {
         const float a = fabsf(xv);
+        const bool n = xv < 0.0f;
         if (a < min0) {
             min1 = min0;
             a1 = a0;
+            n1 = n0;
             min0 = a;
             a0 = k;
+            n0 = n;
         } else if (a < min1) {
             min1 = a;
             a1 = k;
+            n1 = n;
         }
-        neg ^= xv < 0.0f;
+        neg ^= n;
     }
-    for (int k = 0; k < D; k++) {
-        if (k == 1 && !has_pp)
-            continue;
-        const float muraw = k == a0 ? min1 : min0;
-        const float mu = fminf(muraw, 127.0f);
-        const float pre = beta * mu - alpha;
-        const float mag = fmaxf(pre, 0.0f);
-        const bool sneg = neg ^ (x[k] < 0.0f);
-        const float sg = sneg ? -1.0f : 1.0f;
-        const float m = sg * mag;
-        const size_t e = (size_t)k * c.R + slotpos;
-        const float gpo = s.gP[var[k]];       /* d L / d P' */
-        const float gmo = s.gM ? s.gM[e] : 0; /* d L / d stored message */
-        const float post = x[k] + m;
-        const float gpost = (post >= -128.0f && post <= 127.0f) ? gpo : 0.0f;
-        const float gmsg = (m >= -32.0f && m <= 31.0f) ? gmo : 0.0f;
-        const float gm = gpost + gmsg;
-        gx[k] += gpost;
-        if (pre > 0.0f) {
-            const float gmag = gm * sg;
-            dbeta += gmag * mu;
-            dalpha -= gmag;
-            if (muraw < 127.0f) {
-                const int src = k == a0 ? a1 : a0;
-                gx[src] += gmag * beta * (x[src] < 0.0f ? -1.0f : 1.0f);
-            }
-        }
-    }
-    for (int k = 0; k < D; k++) {
-        if (k == 1 && !has_pp)
-            continue;
-        const bool inside = raw[k] >= -128.0f && raw[k] <= 127.0f;
-        const float g = inside ? gx[k] : 0.0f;
-        s.gP[var[k]] = g;
-        if (s.gM)
-            s.gM[(size_t)k * c.R + slotpos] = first ? 0.0f : -g;
-    }
-}
+};
 
-/* One iteration (all steps), forward. */
-__device__ void iteration_fwd(const DevCode& c, const LFrame& s, const LearnedParams& p, int t,
-                              const float* sbeta, const float* salpha)
-{
-    const int tid = threadIdx.x;
-    for (int st_i = 0; st_i < c.nsteps; st_i++) {
-        const uint32_t st = c.steps[st_i];
-        const int i = st & 0xFF, start = (st >> 8) & 0x1FF, n = (st >> 17) & 0x1FF;
-        for (int g = tid; g < n; g += blockDim.x) {
-            const int pos = start + g;
-            const int j = (st >> 26) ? (int)c.perm[kQCl * i + pos] : pos;
-            const int D = c.eoff[i + 1] - c.eoff[i] + 2 - ((i | j) ? 0 : 1);
-            const int k = p.cls[D];
-            check_fwd(c, s, i, j, kQCl * i + pos, sbeta[k], salpha[k], t == 0);
-        }
-        __syncthreads();
-    }
-}
-
-/* Loss of the posteriors after iteration t; optionally its gradient into gP. */
-__device__ float iteration_loss(const DevCode& c, const LFrame& s, const LearnedParams& p, int f, float gscale)
+/* Loss of the posteriors after an iteration (and a copy of them). */
+__device__ float iteration_loss(const DevCode& c, const float* __restrict__ P, const LearnedParams& p, int f,
+                                float* __restrict__ copy)
 {
     const uint8_t* bits = p.bits + (size_t)f * p.bits_stride;
     float acc = 0.0f;
     for (int v = threadIdx.x; v < c.kldpc; v += blockDim.x) {
         const float sb = ((bits[v >> 3] >> (7 - (v & 7))) & 1) ? -1.0f : 1.0f; /* +1 for a 0 bit */
-        const float u = -sb * s.P[v] * 0.5f;
-        acc += softplus(u);
-        if (gscale != 0.0f)
-            s.gP[v] += gscale * (-sb * 0.5f) * sigmoid(u);
+        const float x = P[v];
+        if (copy)
+            __stcs(copy + v, x);
+        acc += softplus(-sb * x * 0.5f);
     }
     return acc;
 }
@@ -254,122 +151,277 @@ __device__ void load_params(const LearnedParams& p, int t, float* sbeta, float* 
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(kLT) k_learned_fwd(LearnedParams p)
+/* Bound by instruction issue (about 90 a link forward) and, in the layers with
+ * wavefront levels, by the warps that wait for a level's few; DRAM 12 %, L2 hits
+ * two thirds.  512 normal 2/3 frames, 20 iterations, loss and gradients: 219 ->
+ * 73.5 ms.  Before, the backward pass ran every iteration again from a
+ * checkpoint of posteriors and messages, and a check's links were arrays
+ * indexed at run time, in local memory. */
+
+/* resident CTAs per SM that a degree bound's registers are compiled for */
+__host__ __device__ constexpr int fwd_ctas(int dm) { return dm <= 11 ? 3 : dm <= 22 ? 2 : 1; }
+__host__ __device__ constexpr int bwd_ctas(int dm) { return dm <= 18 ? 2 : 1; }
+
+template <int DM, bool TRAIN>
+__global__ void __launch_bounds__(kLT, fwd_ctas(DM)) k_learned_fwd(LearnedParams p)
 {
+    extern __shared__ __align__(16) char smem[];
     __shared__ float sbeta[kLearnedMaxClass], salpha[kLearnedMaxClass], red[kLT / 32];
-    const DevCode& c = *p.code;
-    const int f = blockIdx.x;
-    const LFrame s = frame_state(p, f);
+    const DevCode c = *p.code;
+    const LTables tb = stage_tables(c, smem);
+    const int f = blockIdx.x, j = threadIdx.x;
+    const bool active = j < kQCl;
     const size_t E = (size_t)p.DS * c.R;
+    float* P = p.P + (size_t)f * c.N;
+    uint4* M = p.M + (size_t)f * c.R;
     const __half* src = p.llr + (size_t)f * p.llr_stride;
-    for (int v = threadIdx.x; v < c.K; v += blockDim.x)
-        s.P[v] = clampf(__half2float(src[v]), -128.0f, 127.0f);
-    for (int k = threadIdx.x; k < c.R; k += blockDim.x)
-        s.P[c.K + kQCl * (k % c.q) + k / c.q] = clampf(__half2float(src[c.K + k]), -128.0f, 127.0f);
+    for (int v = j; v < c.K; v += blockDim.x)
+        P[v] = clampf(__half2float(src[v]), -128.0f, 127.0f);
+    for (int k = j; k < c.R; k += blockDim.x)
+        P[c.K + kQCl * (k % c.q) + k / c.q] = clampf(__half2float(src[c.K + k]), -128.0f, 127.0f);
     __syncthreads();
     for (int t = 0; t < p.iters; t++) {
-        if (p.Pck) {
-            float* pc = p.Pck + ((size_t)t * p.nframes + f) * c.N;
-            float* mc = p.Mck + ((size_t)t * p.nframes + f) * E;
-            for (int v = threadIdx.x; v < c.N; v += blockDim.x)
-                pc[v] = s.P[v];
-            if (t > 0)
-                for (size_t e = threadIdx.x; e < E; e += blockDim.x)
-                    mc[e] = s.M[e];
-        }
         load_params(p, t, sbeta, salpha);
-        LFrame sf = s;
-        sf.X = nullptr;
-        iteration_fwd(c, sf, p, t, sbeta, salpha);
-        const float l = block_sum(iteration_loss(c, s, p, f, 0.0f), red);
-        if (threadIdx.x == 0)
+        float* X = TRAIN ? p.Xck + ((size_t)t * p.nframes + f) * E : nullptr;
+        uint4 rn = make_uint4(0, 0, 0, 0); /* records and levels one layer ahead */
+        unsigned long long mn = 0;
+        if (active) {
+            if (t)
+                rn = M[j];
+            mn = __ldg(c.lmeta + j);
+        }
+        for (int i = 0; i < c.q; i++) {
+            const uint4 rec = rn;
+            const unsigned long long meta = mn;
+            if (active && i + 1 < c.q) {
+                if (t)
+                    rn = M[kQCl * (i + 1) + j];
+                mn = __ldg(c.lmeta + kQCl * (i + 1) + j);
+            }
+            const int2* ent = tb.ent + tb.eoff[i];
+            const int D = tb.eoff[i + 1] - tb.eoff[i] + 2, nl = tb.nlev[i], pos = kQCl * i + j;
+            const uint32_t live = ((i | j) ? 0xFFFFFFFFu : ~2u) & (D < 32 ? (1u << D) - 1u : 0xFFFFFFFFu);
+            const uint32_t late = (uint32_t)(meta >> 8) & 0xFFFFFFu;
+            const int lev = (int)(meta & 0xFF);
+            float raw[DM];
+            auto load = [&](int k) {
+                /* the link's old message */
+                const float mag = (int)rec.w == k ? __uint_as_float(rec.y) : __uint_as_float(rec.x);
+                const float m = clampf((rec.z >> k) & 1u ? -mag : mag, -32.0f, 31.0f);
+                raw[k] = P[link_var(c, ent, i, j, k)] - (t == 0 ? 0.0f : m);
+            };
+            if (active) {
+#pragma unroll
+                for (int k = 0; k < DM; k++)
+                    if (((live & ~late) >> k) & 1u)
+                        load(k);
+            }
+            for (int l = 0; l < nl; l++) {
+                if (active && lev == l) {
+                    if (late) {
+#pragma unroll
+                        for (int k = 2; k < DM; k++)
+                            if ((late >> k) & 1u)
+                                load(k);
+                    }
+                    Node n;
+#pragma unroll
+                    for (int k = 0; k < DM; k++)
+                        if ((live >> k) & 1u)
+                            n.add(clampf(raw[k], -128.0f, 127.0f), k);
+                    const int cl = p.cls[D - ((i | j) ? 0 : 1)];
+                    const float beta = sbeta[cl], alpha = salpha[cl];
+                    const float mu0 = fminf(n.min0, 127.0f), mu1 = fminf(n.min1, 127.0f);
+                    const float mag0 = fmaxf(beta * mu0 - alpha, 0.0f), mag1 = fmaxf(beta * mu1 - alpha, 0.0f);
+                    uint32_t signs = 0;
+#pragma unroll
+                    for (int k = 0; k < DM; k++)
+                        if ((live >> k) & 1u) {
+                            const float x = clampf(raw[k], -128.0f, 127.0f);
+                            const float mag = k == n.a0 ? mag1 : mag0;
+                            const bool sneg = n.neg ^ (x < 0.0f);
+                            signs |= sneg ? 1u << k : 0u;
+                            P[link_var(c, ent, i, j, k)] = clampf(x + (sneg ? -mag : mag), -128.0f, 127.0f);
+                            if (TRAIN)
+                                __stcs(X + (size_t)k * c.R + pos, raw[k]);
+                        }
+                    M[pos] = make_uint4(__float_as_uint(mag0), __float_as_uint(mag1), signs, (uint32_t)n.a0);
+                }
+                __syncthreads();
+            }
+        }
+        float* copy = TRAIN ? p.Pck + ((size_t)t * p.nframes + f) * c.K : nullptr;
+        const float l = block_sum(iteration_loss(c, P, p, f, copy), red);
+        if (j == 0)
             atomicAdd(p.loss + t, l);
     }
     if (p.post)
-        for (int v = threadIdx.x; v < c.kldpc; v += blockDim.x)
-            p.post[(size_t)f * c.kldpc + v] = s.P[v];
+        for (int v = j; v < c.kldpc; v += blockDim.x)
+            p.post[(size_t)f * c.kldpc + v] = P[v];
 }
 
-__global__ void __launch_bounds__(kLT) k_learned_bwd(LearnedParams p)
+template <int DM>
+__global__ void __launch_bounds__(kLT, bwd_ctas(DM)) k_learned_bwd(LearnedParams p)
 {
-    __shared__ float sbeta[kLearnedMaxClass], salpha[kLearnedMaxClass], red[kLT / 32];
+    extern __shared__ __align__(16) char smem[];
+    __shared__ float sbeta[kLearnedMaxClass], salpha[kLearnedMaxClass];
     __shared__ float sdb[kLearnedMaxClass], sda[kLearnedMaxClass];
-    const DevCode& c = *p.code;
-    const int f = blockIdx.x;
-    const LFrame s = frame_state(p, f);
+    const DevCode c = *p.code;
+    const LTables tb = stage_tables(c, smem);
+    const int f = blockIdx.x, j = threadIdx.x, lane = j & 31;
+    const bool active = j < kQCl;
     const size_t E = (size_t)p.DS * c.R;
-    for (int v = threadIdx.x; v < c.N; v += blockDim.x)
-        s.gP[v] = 0.0f;
-    for (size_t e = threadIdx.x; e < E; e += blockDim.x)
-        s.gM[e] = 0.0f;
-    __syncthreads();
+    float* gP = p.gP + (size_t)f * c.N;
+    float* gM = p.gM + (size_t)f * E;
+    const uint8_t* bits = p.bits + (size_t)f * p.bits_stride;
     for (int t = p.iters - 1; t >= 0; t--) {
-        /* restore the state at the start of iteration t */
-        const float* pc = p.Pck + ((size_t)t * p.nframes + f) * c.N;
-        const float* mc = p.Mck + ((size_t)t * p.nframes + f) * E;
-        for (int v = threadIdx.x; v < c.N; v += blockDim.x)
-            s.P[v] = pc[v];
-        if (t > 0)
-            for (size_t e = threadIdx.x; e < E; e += blockDim.x)
-                s.M[e] = mc[e];
-        if ((int)threadIdx.x < kLearnedMaxClass) {
-            sdb[threadIdx.x] = 0.0f;
-            sda[threadIdx.x] = 0.0f;
-        }
+        const bool lastit = t == p.iters - 1;
+        if (j < kLearnedMaxClass)
+            sdb[j] = sda[j] = 0.0f;
         load_params(p, t, sbeta, salpha);
-        iteration_fwd(c, s, p, t, sbeta, salpha); /* saves X */
-        iteration_loss(c, s, p, f, p.loss_scale * (p.loss_w ? p.loss_w[t] : 1.0f));
+        /* the gradient of the iteration's loss */
+        const float* P = p.Pck + ((size_t)t * p.nframes + f) * c.K;
+        const float* X = p.Xck + ((size_t)t * p.nframes + f) * E;
+        const float gscale = p.loss_scale * (p.loss_w ? p.loss_w[t] : 1.0f);
+        for (int v = j; v < (lastit ? c.N : c.kldpc); v += blockDim.x) {
+            float g = 0.0f;
+            if (v < c.kldpc) {
+                const float sb = ((bits[v >> 3] >> (7 - (v & 7))) & 1) ? -1.0f : 1.0f;
+                g = gscale * (-sb * 0.5f) * sigmoid(-sb * __ldcs(P + v) * 0.5f);
+            }
+            gP[v] = lastit ? g : gP[v] + g;
+        }
         __syncthreads();
-        float db[kLearnedMaxClass], da[kLearnedMaxClass];
-        for (int k = 0; k < p.nclass; k++)
-            db[k] = da[k] = 0.0f;
-        for (int st_i = c.nsteps - 1; st_i >= 0; st_i--) {
-            const uint32_t st = c.steps[st_i];
-            const int i = st & 0xFF, start = (st >> 8) & 0x1FF, n = (st >> 17) & 0x1FF;
-            for (int g = threadIdx.x; g < n; g += blockDim.x) {
-                const int pos = start + g;
-                const int j = (st >> 26) ? (int)c.perm[kQCl * i + pos] : pos;
-                const int D = c.eoff[i + 1] - c.eoff[i] + 2 - ((i | j) ? 0 : 1);
-                const int k = p.cls[D];
-                float b = 0.0f, a = 0.0f;
-                check_bwd(c, s, i, j, kQCl * i + pos, sbeta[k], salpha[k], t == 0, b, a);
-                for (int kk = 0; kk < p.nclass; kk++)
-                    if (kk == k) {
-                        db[kk] += b;
-                        da[kk] += a;
+        float db = 0.0f, da = 0.0f; /* of the layers' class since the last flush */
+        for (int i = c.q - 1; i >= 0; i--) {
+            const int2* ent = tb.ent + tb.eoff[i];
+            const int D = tb.eoff[i + 1] - tb.eoff[i] + 2, nl = tb.nlev[i], pos = kQCl * i + j;
+            const uint32_t live = ((i | j) ? 0xFFFFFFFFu : ~2u) & (D < 32 ? (1u << D) - 1u : 0xFFFFFFFFu);
+            float raw[DM], go[DM], gmo[DM];
+            uint32_t early = 0;
+            int lev = 0;
+            if (active) {
+                const unsigned long long meta = __ldg(c.lmeta + pos);
+                early = (uint32_t)(meta >> 32) & 0xFFFFFFu; /* outputs that later checks of the layer read */
+                lev = (int)(meta & 0xFF);
+#pragma unroll
+                for (int k = 0; k < DM; k++)
+                    if ((live >> k) & 1u) {
+                        raw[k] = __ldcs(X + (size_t)k * c.R + pos);
+                        gmo[k] = lastit ? 0.0f : __ldcs(gM + (size_t)k * c.R + pos);
+                        if (!((early >> k) & 1u))
+                            go[k] = gP[link_var(c, ent, i, j, k)];
                     }
             }
-            __syncthreads();
-        }
-        for (int k = 0; k < p.nclass; k++) {
-            const float b = block_sum(db[k], red), a = block_sum(da[k], red);
-            if (threadIdx.x == 0) {
-                atomicAdd(p.dbeta + t * p.nclass + k, b);
-                atomicAdd(p.dalpha + t * p.nclass + k, a);
+            for (int l = nl - 1; l >= 0; l--) {
+                if (active && lev == l) {
+                    if (early) {
+#pragma unroll
+                        for (int k = 2; k < DM; k++)
+                            if ((early >> k) & 1u)
+                                go[k] = gP[link_var(c, ent, i, j, k)];
+                    }
+                    Node n;
+#pragma unroll
+                    for (int k = 0; k < DM; k++)
+                        if ((live >> k) & 1u)
+                            n.add(clampf(raw[k], -128.0f, 127.0f), k);
+                    const int cl = p.cls[D - ((i | j) ? 0 : 1)];
+                    const float beta = sbeta[cl], alpha = salpha[cl];
+                    const float mu0 = fminf(n.min0, 127.0f), mu1 = fminf(n.min1, 127.0f);
+                    const float pre0 = beta * mu0 - alpha, pre1 = beta * mu1 - alpha;
+                    const float mag0 = fmaxf(pre0, 0.0f), mag1 = fmaxf(pre1, 0.0f);
+                    float s0 = 0.0f, s1 = 0.0f, b = 0.0f, a = 0.0f; /* to the links of the minimums, scale, offset */
+#pragma unroll
+                    for (int k = 0; k < DM; k++)
+                        if ((live >> k) & 1u) {
+                            const float x = clampf(raw[k], -128.0f, 127.0f);
+                            const bool own = k == n.a0;
+                            const bool sneg = n.neg ^ (x < 0.0f);
+                            const float mag = own ? mag1 : mag0, m = sneg ? -mag : mag;
+                            const float post = x + m;
+                            const float gpost = (post >= -128.0f && post <= 127.0f) ? go[k] : 0.0f;
+                            const float gmsg = (m >= -32.0f && m <= 31.0f) ? gmo[k] : 0.0f;
+                            const float gm = gpost + gmsg, gmag = sneg ? -gm : gm;
+                            go[k] = gpost;
+                            if ((own ? pre1 : pre0) > 0.0f) {
+                                b += gmag * (own ? mu1 : mu0);
+                                a -= gmag;
+                                if (own)
+                                    s1 = gmag;
+                                else
+                                    s0 += gmag;
+                            }
+                        }
+                    s0 = n.min0 < 127.0f ? s0 * beta * (n.n0 ? -1.0f : 1.0f) : 0.0f;
+                    s1 = n.min1 < 127.0f ? s1 * beta * (n.n1 ? -1.0f : 1.0f) : 0.0f;
+#pragma unroll
+                    for (int k = 0; k < DM; k++)
+                        if ((live >> k) & 1u) {
+                            const bool inside = raw[k] >= -128.0f && raw[k] <= 127.0f;
+                            const float gx = go[k] + (k == n.a0 ? s0 : k == n.a1 ? s1 : 0.0f);
+                            const float g = inside ? gx : 0.0f;
+                            gP[link_var(c, ent, i, j, k)] = g;
+                            if (t)
+                                __stcs(gM + (size_t)k * c.R + pos, -g);
+                        }
+                    if (i | j) {
+                        db += b;
+                        da += a;
+                    } else { /* the one check of another degree */
+                        atomicAdd(sdb + cl, b);
+                        atomicAdd(sda + cl, a);
+                    }
+                }
+                __syncthreads();
+            }
+            /* the sums leave the registers where the layers' degree changes */
+            if (i == 0 || tb.eoff[i] - tb.eoff[i - 1] != D - 2) {
+                for (int o = 16; o > 0; o >>= 1) {
+                    db += __shfl_xor_sync(0xFFFFFFFFu, db, o);
+                    da += __shfl_xor_sync(0xFFFFFFFFu, da, o);
+                }
+                if (lane == 0) {
+                    atomicAdd(sdb + p.cls[D], db);
+                    atomicAdd(sda + p.cls[D], da);
+                }
+                db = da = 0.0f;
             }
         }
+        __syncthreads();
+        if (j < p.nclass) {
+            atomicAdd(p.dbeta + t * p.nclass + j, sdb[j]);
+            atomicAdd(p.dalpha + t * p.nclass + j, sda[j]);
+        }
+        __syncthreads();
     }
 }
 
-size_t learned_workspace_bytes(const DevCode& host_code_shape, int R, int N, int DS, int nframes, int iters,
-                               bool train)
-{
-    (void)host_code_shape;
-    const size_t E = (size_t)DS * R;
-    size_t b = (size_t)nframes * (N + E) * sizeof(float); /* P, M */
-    if (train)
-        b += (size_t)nframes * (N + 2 * E) * sizeof(float) +          /* gP, gM, X */
-             (size_t)iters * nframes * (N + E) * sizeof(float);        /* checkpoints */
-    return b;
-}
-
-cudaError_t launch_learned(const LearnedParams& p, bool backward, cudaStream_t s)
+template <int DM>
+static cudaError_t launch_degree(const LearnedParams& p, bool backward, size_t smem, cudaStream_t s)
 {
     if (backward)
-        k_learned_bwd<<<p.nframes, kLT, 0, s>>>(p);
+        k_learned_bwd<DM><<<p.nframes, kLT, smem, s>>>(p);
+    else if (p.Xck)
+        k_learned_fwd<DM, true><<<p.nframes, kLT, smem, s>>>(p);
     else
-        k_learned_fwd<<<p.nframes, kLT, 0, s>>>(p);
+        k_learned_fwd<DM, false><<<p.nframes, kLT, smem, s>>>(p);
     return cudaGetLastError();
+}
+
+cudaError_t launch_learned(const LearnedParams& p, bool backward, int dclass, int nent, int q, cudaStream_t s)
+{
+    const size_t smem = sizeof(int2) * (size_t)nent + sizeof(uint16_t) * (q + 1) + q;
+    static_assert(kNumClasses == 6 && kClassDeg[5] == 32, "degree classes");
+    switch (dclass) {
+    case 0: return launch_degree<kClassDeg[0]>(p, backward, smem, s);
+    case 1: return launch_degree<kClassDeg[1]>(p, backward, smem, s);
+    case 2: return launch_degree<kClassDeg[2]>(p, backward, smem, s);
+    case 3: return launch_degree<kClassDeg[3]>(p, backward, smem, s);
+    case 4: return launch_degree<kClassDeg[4]>(p, backward, smem, s);
+    case 5: return launch_degree<kClassDeg[5]>(p, backward, smem, s);
+    }
+    return cudaErrorInvalidValue;
 }
 
 }  // namespace drxg

@@ -29,12 +29,11 @@ struct LearnedParams {
     int nclass;
     const int8_t* cls;   /* class of each check degree 0..32 (device) */
     float* P;            /* workspace: nframes x N posteriors */
-    float* M;            /* nframes x DS*R messages */
-    float* X;            /* backward: nframes x DS*R extrinsic inputs */
+    uint4* M;            /* nframes x R message records */
     float* gP;           /* backward: nframes x N */
     float* gM;           /* backward: nframes x DS*R */
-    float* Pck;          /* training: iters x nframes x N checkpoints (null: none) */
-    float* Mck;          /* iters x nframes x DS*R */
+    float* Pck;          /* training: iters x nframes x K posteriors after each iteration (null: none) */
+    float* Xck;          /* iters x nframes x DS*R extrinsic inputs (slot-major) */
     float* loss;         /* iters: sums of the BCE of every iteration's output */
     float* dbeta;        /* backward: iters x nclass */
     float* dalpha;
@@ -43,8 +42,7 @@ struct LearnedParams {
     float* post;         /* forward, optional: nframes x kldpc final posteriors */
 };
 
-size_t learned_workspace_bytes(const DevCode& host_code_shape, int R, int N, int DS, int nframes, int iters,
-                               bool train);
-cudaError_t launch_learned(const LearnedParams& p, bool backward, cudaStream_t s);
+/* dclass, nent, q: the code's degree class, information entries and layers */
+cudaError_t launch_learned(const LearnedParams& p, bool backward, int dclass, int nent, int q, cudaStream_t s);
 
 }  // namespace drxg

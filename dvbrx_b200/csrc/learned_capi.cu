@@ -5,8 +5,9 @@
  * The caller owns all memory: a workspace sized by
  * drx_learned_workspace_bytes, the per-iteration loss sums and the gradient
  * accumulators.  Workspace layout: 64 bytes of check-degree classes, then
- * (16-byte aligned) P, M, and for training X, gP, gM, the P checkpoints and
- * the message checkpoints, all fp32.
+ * (16-byte aligned) the posteriors (fp32) and the message records, and for
+ * training gP, gM, and of every iteration the information posteriors after it
+ * and the extrinsic inputs, all fp32.
  */
 #include <cuda_runtime.h>
 #include <string.h>
@@ -24,12 +25,12 @@ namespace {
 size_t a16(size_t v) { return (v + 15) & ~(size_t)15; }
 
 struct WsLayout {
-    size_t cls, P, M, X, gP, gM, Pck, Mck, total;
+    size_t cls, P, M, gP, gM, Pck, Xck, total;
 };
 
 WsLayout layout(const drx_ldpc* d, int nframes, int iters, bool train)
 {
-    const size_t N = d->code.N, E = (size_t)d->code.deg_max * d->code.R, F = nframes;
+    const size_t N = d->code.N, K = d->code.K, R = d->code.R, E = d->code.deg_max * R, F = nframes;
     WsLayout w{};
     size_t off = 0;
     w.cls = off;
@@ -37,17 +38,15 @@ WsLayout layout(const drx_ldpc* d, int nframes, int iters, bool train)
     w.P = off;
     off = a16(off + F * N * 4);
     w.M = off;
-    off = a16(off + F * E * 4);
+    off = a16(off + F * R * sizeof(uint4));
     if (train) {
-        w.X = off;
-        off = a16(off + F * E * 4);
         w.gP = off;
         off = a16(off + F * N * 4);
         w.gM = off;
         off = a16(off + F * E * 4);
         w.Pck = off;
-        off = a16(off + (size_t)iters * F * N * 4);
-        w.Mck = off;
+        off = a16(off + (size_t)iters * F * K * 4);
+        w.Xck = off;
         off = a16(off + (size_t)iters * F * E * 4);
     }
     w.total = off;
@@ -62,7 +61,7 @@ int fill(drx_ldpc* d, LearnedParams& p, int nframes, const void* llr, size_t llr
         set_error("learned decoder: bad arguments");
         return -1;
     }
-    if (nclass < 1 || nclass > kLearnedMaxClass || d->code.deg_max > kLearnedMaxDeg) {
+    if (nclass < 1 || nclass > kLearnedMaxClass || d->code.deg_max > kLearnedMaxDeg || !d->code.phased) {
         set_error("learned decoder: unsupported class count or degree");
         return -1;
     }
@@ -97,15 +96,19 @@ int fill(drx_ldpc* d, LearnedParams& p, int nframes, const void* llr, size_t llr
     p.nclass = nclass;
     p.cls = (const int8_t*)(b + w.cls);
     p.P = (float*)(b + w.P);
-    p.M = (float*)(b + w.M);
+    p.M = (uint4*)(b + w.M);
     if (train) {
-        p.X = (float*)(b + w.X);
         p.gP = (float*)(b + w.gP);
         p.gM = (float*)(b + w.gM);
         p.Pck = (float*)(b + w.Pck);
-        p.Mck = (float*)(b + w.Mck);
+        p.Xck = (float*)(b + w.Xck);
     }
     return 0;
+}
+
+cudaError_t launch(const drx_ldpc* d, const LearnedParams& p, bool backward, cudaStream_t s)
+{
+    return launch_learned(p, backward, d->code.dclass, (int)d->code.ent.size() / 2, d->code.q, s);
 }
 
 }  // namespace
@@ -135,7 +138,7 @@ int drx_learned_forward(drx_ldpc* d, int nframes, const void* llr_f16, size_t ll
     }
     p.loss = loss;
     p.post = post;
-    return cuda_check(launch_learned(p, false, s), "learned forward") ? 0 : -1;
+    return cuda_check(launch(d, p, false, s), "learned forward") ? 0 : -1;
 }
 
 int drx_learned_backward(drx_ldpc* d, int nframes, const void* llr_f16, size_t llr_stride, const uint8_t* bits,
@@ -158,7 +161,7 @@ int drx_learned_backward(drx_ldpc* d, int nframes, const void* llr_f16, size_t l
     p.loss_w = iter_weights;
     p.dbeta = dbeta;
     p.dalpha = dalpha;
-    return cuda_check(launch_learned(p, true, s), "learned backward") ? 0 : -1;
+    return cuda_check(launch(d, p, true, s), "learned backward") ? 0 : -1;
 }
 
 int drx_ldpc_schedule(int short_frame, const char* rate, int* nsteps, int* deg_max, int32_t* check_step,

@@ -12,9 +12,9 @@ on the int8 decoder's scale (2 x LLR) with its saturations, evaluated in fp32
 binary cross-entropy of the information bits after every iteration.
 
 ``LearnedMinSum`` is the ``torch.autograd.Function``: its forward runs
-``drx_learned_forward`` keeping one checkpoint of the decoder state per
-iteration, its backward runs ``drx_learned_backward``, which re-runs each
-iteration from its checkpoint and walks it in reverse.  ``LearnedDecoder`` is
+``drx_learned_forward`` keeping every iteration's extrinsic inputs, its
+backward runs ``drx_learned_backward``, which walks each iteration in reverse
+from them.  ``LearnedDecoder`` is
 the module with fp32 master parameters.
 """
 import ctypes

@@ -251,7 +251,8 @@ size_t drx_learned_workspace_bytes(const drx_ldpc* d, int nframes, int iters, in
 /* Forward over nframes frames; loss[t] (device, zeroed by the caller)
  * receives the BCE sum after iteration t; post (device, optional) the final
  * posteriors of the kldpc information bits.  With train != 0 the
- * workspace keeps one checkpoint per iteration for drx_learned_backward. */
+ * workspace keeps every iteration's extrinsic inputs and posteriors for
+ * drx_learned_backward. */
 int drx_learned_forward(drx_ldpc* d, int nframes, const void* llr_f16, size_t llr_stride, const uint8_t* bits,
                         size_t bits_stride, int iters, const void* beta_f16, const void* alpha_f16, int nclass,
                         const int8_t* class_of_degree, float* loss, float* post, void* workspace,
