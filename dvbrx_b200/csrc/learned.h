@@ -7,6 +7,7 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include "codes.h"
 #include "ldpc_device.h"
 
 namespace drxg {
@@ -31,9 +32,9 @@ struct LearnedParams {
     float* P;            /* workspace: nframes x N posteriors */
     uint4* M;            /* nframes x R message records */
     float* gP;           /* backward: nframes x N */
-    float* gM;           /* backward: nframes x DS*R */
+    float* gM;           /* backward: nframes x DS*R (layer, slot, check) */
     float* Pck;          /* training: iters x nframes x K posteriors after each iteration (null: none) */
-    float* Xck;          /* iters x nframes x DS*R extrinsic inputs (slot-major) */
+    float* Xck;          /* iters x nframes x DS*R extrinsic inputs (layer, slot, check) */
     float* loss;         /* iters: sums of the BCE of every iteration's output */
     float* dbeta;        /* backward: iters x nclass */
     float* dalpha;
@@ -42,7 +43,6 @@ struct LearnedParams {
     float* post;         /* forward, optional: nframes x kldpc final posteriors */
 };
 
-/* dclass, nent, q: the code's degree class, information entries and layers */
-cudaError_t launch_learned(const LearnedParams& p, bool backward, int dclass, int nent, int q, cudaStream_t s);
+cudaError_t launch_learned(const LearnedParams& p, bool backward, const Code& code, cudaStream_t s);
 
 }  // namespace drxg

@@ -106,11 +106,6 @@ int fill(drx_ldpc* d, LearnedParams& p, int nframes, const void* llr, size_t llr
     return 0;
 }
 
-cudaError_t launch(const drx_ldpc* d, const LearnedParams& p, bool backward, cudaStream_t s)
-{
-    return launch_learned(p, backward, d->code.dclass, (int)d->code.ent.size() / 2, d->code.q, s);
-}
-
 }  // namespace
 
 extern "C" {
@@ -138,7 +133,7 @@ int drx_learned_forward(drx_ldpc* d, int nframes, const void* llr_f16, size_t ll
     }
     p.loss = loss;
     p.post = post;
-    return cuda_check(launch(d, p, false, s), "learned forward") ? 0 : -1;
+    return cuda_check(launch_learned(p, false, d->code, s), "learned forward") ? 0 : -1;
 }
 
 int drx_learned_backward(drx_ldpc* d, int nframes, const void* llr_f16, size_t llr_stride, const uint8_t* bits,
@@ -161,7 +156,7 @@ int drx_learned_backward(drx_ldpc* d, int nframes, const void* llr_f16, size_t l
     p.loss_w = iter_weights;
     p.dbeta = dbeta;
     p.dalpha = dalpha;
-    return cuda_check(launch(d, p, true, s), "learned backward") ? 0 : -1;
+    return cuda_check(launch_learned(p, true, d->code, s), "learned backward") ? 0 : -1;
 }
 
 int drx_ldpc_schedule(int short_frame, const char* rate, int* nsteps, int* deg_max, int32_t* check_step,
