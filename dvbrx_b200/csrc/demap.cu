@@ -59,15 +59,45 @@ struct DemapParams {
     int nframes;
 };
 
-__device__ __forceinline__ int8_t quantise8(float v)
+/* v clamped to +-127 and rounded half to even, in the low byte: the sum with
+ * 1.5 2^23 rounds so, and its low bits are the integer's (a conversion
+ * instruction issues at a quarter of the rate) */
+__device__ __forceinline__ uint32_t quantise8(float v)
 {
     v = fminf(fmaxf(v, -127.0f), 127.0f);
-    return (int8_t)__float2int_rn(v);
+    return __float_as_uint(__fadd_rn(v, 12582912.0f));
 }
 
-/* LLRs of one symbol, label bit b in out[b] */
+/* the low bytes of four words */
+__device__ __forceinline__ uint32_t pack4(uint32_t a, uint32_t b, uint32_t c, uint32_t d)
+{
+    return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
+}
+
+/* Minima of 2^BITS distances over the points whose index has bit L clear (lo[L])
+ * and set (hi[L]): the pairs that differ in the lowest bit, then their minima
+ * as half as many distances (v is overwritten; v[0] is the minimum of all). */
 template <int BITS>
-__device__ __forceinline__ void demap_symbol(const DemapParams& p, float x, float y, float k, int8_t* out)
+__device__ __forceinline__ void bit_minima(float* v, float* lo, float* hi)
+{
+#pragma unroll
+    for (int L = 0, n = 1 << BITS; L < BITS; L++, n /= 2) {
+        lo[L] = v[0];
+        hi[L] = v[1];
+#pragma unroll
+        for (int q = 2; q < n; q += 2) {
+            lo[L] = fminf(lo[L], v[q]);
+            hi[L] = fminf(hi[L], v[q + 1]);
+        }
+#pragma unroll
+        for (int q = 0; q < n / 2; q++)
+            v[q] = fminf(v[2 * q], v[2 * q + 1]);
+    }
+}
+
+/* LLRs of one symbol, label bit b in the low byte of out[b] */
+template <int BITS>
+__device__ __forceinline__ void demap_symbol(const DemapParams& p, float x, float y, float k, uint32_t* out)
 {
     if (BITS == 2) {
         const float kq = k * 4.0f * 0.70710678118654752f; /* demap.c:496-500 */
@@ -127,25 +157,14 @@ __device__ __forceinline__ void demap_symbol(const DemapParams& p, float x, floa
                 const int pt = 16 * g + q;
                 v[q] = fmaf(x, p.ar[pt], fmaf(y, p.ai[pt], p.e[pt]));
             }
-            float t[16];
+            float lo[4], hi[4];
+            bit_minima<4>(v, lo, hi);
 #pragma unroll
-            for (int q = 0; q < 16; q++)
-                t[q] = v[q];
-#pragma unroll
-            for (int L = 0, n = 16; L < 4; L++, n /= 2) {
-                float lo = t[0], hi = t[1];
-#pragma unroll
-                for (int q = 2; q < n; q += 2) {
-                    lo = fminf(lo, t[q]);
-                    hi = fminf(hi, t[q + 1]);
-                }
-                m0[BITS - 1 - L] = fminf(m0[BITS - 1 - L], lo);
-                m1[BITS - 1 - L] = fminf(m1[BITS - 1 - L], hi);
-#pragma unroll
-                for (int q = 0; q < n / 2; q++)
-                    t[q] = fminf(t[2 * q], t[2 * q + 1]);
+            for (int L = 0; L < 4; L++) {
+                m0[BITS - 1 - L] = fminf(m0[BITS - 1 - L], lo[L]);
+                m1[BITS - 1 - L] = fminf(m1[BITS - 1 - L], hi[L]);
             }
-            gmin[g] = t[0];
+            gmin[g] = v[0];
         }
 #pragma unroll
         for (int L = 4; L < BITS; L++) {
@@ -162,16 +181,15 @@ __device__ __forceinline__ void demap_symbol(const DemapParams& p, float x, floa
         }
         }
     } else {
-#pragma unroll 8
-        for (int q = 0; q < (1 << BITS); q++) {
-            const float d = fmaf(x, p.ar[q], fmaf(y, p.ai[q], p.e[q]));
+        float v[1 << BITS], lo[BITS], hi[BITS];
 #pragma unroll
-            for (int b = 0; b < BITS; b++) {
-                if ((q >> (BITS - 1 - b)) & 1)
-                    m1[b] = fminf(m1[b], d);
-                else
-                    m0[b] = fminf(m0[b], d);
-            }
+        for (int q = 0; q < (1 << BITS); q++)
+            v[q] = fmaf(x, p.ar[q], fmaf(y, p.ai[q], p.e[q]));
+        bit_minima<BITS>(v, lo, hi);
+#pragma unroll
+        for (int L = 0; L < BITS; L++) {
+            m0[BITS - 1 - L] = lo[L];
+            m1[BITS - 1 - L] = hi[L];
         }
     }
 #pragma unroll
@@ -196,29 +214,26 @@ template <int BITS>
 __device__ __forceinline__ void demap_group(const DemapParams& p, const float4& a, const float4& c, int j0, float k,
                                             int8_t* __restrict__ llr)
 {
-    int8_t v[4][BITS];
+    uint32_t v[4][BITS];
     demap_symbol<BITS>(p, a.x, a.y, k, v[0]);
     demap_symbol<BITS>(p, a.z, a.w, k, v[1]);
     demap_symbol<BITS>(p, c.x, c.y, k, v[2]);
     demap_symbol<BITS>(p, c.z, c.w, k, v[3]);
     if (BITS == 2) {
         uint2 w;
-        w.x = (uint32_t)(uint8_t)v[0][0] | (uint32_t)(uint8_t)v[0][1] << 8 | (uint32_t)(uint8_t)v[1][0] << 16 |
-              (uint32_t)(uint8_t)v[1][1] << 24;
-        w.y = (uint32_t)(uint8_t)v[2][0] | (uint32_t)(uint8_t)v[2][1] << 8 | (uint32_t)(uint8_t)v[3][0] << 16 |
-              (uint32_t)(uint8_t)v[3][1] << 24;
+        w.x = pack4(v[0][0], v[0][1], v[1][0], v[1][1]);
+        w.y = pack4(v[2][0], v[2][1], v[3][0], v[3][1]);
         *(uint2*)(llr + 2 * (size_t)j0) = w;
     } else {
 #pragma unroll
         for (int b = 0; b < BITS; b++) {
             const int pos = llr_pos<BITS>(p, b, j0);
             if (pos + 3 < p.nldpc)
-                *(uint32_t*)(llr + pos) = (uint32_t)(uint8_t)v[0][b] | (uint32_t)(uint8_t)v[1][b] << 8 |
-                                          (uint32_t)(uint8_t)v[2][b] << 16 | (uint32_t)(uint8_t)v[3][b] << 24;
+                *(uint32_t*)(llr + pos) = pack4(v[0][b], v[1][b], v[2][b], v[3][b]);
             else
                 for (int s = 0; s < 4; s++)
                     if (pos + s < p.nldpc)
-                        llr[pos + s] = v[s][b];
+                        llr[pos + s] = (int8_t)v[s][b];
         }
     }
 }
@@ -270,7 +285,7 @@ __global__ void __launch_bounds__(256) k_demap(const __grid_constant__ DemapPara
             demap_group<BITS>(p, a, c, j0, k, llr);
         } else {
             const float* sym = p.sym + (size_t)f * p.sym_stride;
-            int8_t v[BITS];
+            uint32_t v[BITS];
             for (int s = 0; s < 4; s++) {
                 const int j = j0 + s;
                 if (j >= p.nsym)
@@ -280,13 +295,68 @@ __global__ void __launch_bounds__(256) k_demap(const __grid_constant__ DemapPara
                 for (int b = 0; b < BITS; b++) {
                     const int pos = llr_pos<BITS>(p, b, j);
                     if (pos < p.nldpc)
-                        llr[pos] = v[b];
+                        llr[pos] = (int8_t)v[b];
                 }
             }
         }
         a = an;
         c = cn;
         vec = vecn;
+    }
+}
+
+/* The same for rows that are all aligned and whole: symbols on 16 bytes, LLRs on
+ * 8, symbol groups of four without a remainder, no padded label bits.  No row is
+ * looked at for its alignment and no store for its end, and the pointers step.
+ * Bound by instruction issue, 225 for four 8PSK symbols of which 186 are the
+ * distances, minimums and roundings (287 in the general kernel): 4096 normal
+ * 8PSK frames 0.218 ms, 68 % of the measured HBM rate; 0.241 in the general
+ * kernel as it was, 0.227 with the minimums from a tree and the rounding by an
+ * addition. */
+template <int BITS>
+__global__ void __launch_bounds__(256) k_demap_rows(const __grid_constant__ DemapParams p)
+{
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    int f = blockIdx.y;
+    if (4 * g >= p.nsym || f >= p.nframes)
+        return;
+    const size_t sym_step = (size_t)gridDim.y * p.sym_stride, llr_step = (size_t)gridDim.y * p.llr_stride;
+    const float* sym = p.sym + (size_t)f * p.sym_stride + 8 * (size_t)g;
+    int8_t* llr = p.llr + (size_t)f * p.llr_stride + 4 * (size_t)g * (BITS == 2 ? 2 : 1);
+    float4 a = __ldcs((const float4*)sym), c = __ldcs((const float4*)sym + 1);
+    float n0 = __ldg(p.n0 + f);
+    while (true) {
+        const int fn = f + gridDim.y;
+        const bool more = fn < p.nframes;
+        float4 an = a, cn = c;
+        float n0n = n0;
+        if (more) {
+            sym += sym_step;
+            an = __ldcs((const float4*)sym);
+            cn = __ldcs((const float4*)sym + 1);
+            n0n = __ldg(p.n0 + fn);
+        }
+        const float k = 2.0f / n0;
+        uint32_t v[4][BITS];
+        demap_symbol<BITS>(p, a.x, a.y, k, v[0]);
+        demap_symbol<BITS>(p, a.z, a.w, k, v[1]);
+        demap_symbol<BITS>(p, c.x, c.y, k, v[2]);
+        demap_symbol<BITS>(p, c.z, c.w, k, v[3]);
+        if (BITS == 2) {
+            *(uint2*)llr = make_uint2(pack4(v[0][0], v[0][1], v[1][0], v[1][1]),
+                                      pack4(v[2][0], v[2][1], v[3][0], v[3][1]));
+        } else {
+#pragma unroll
+            for (int b = 0; b < BITS; b++)
+                *(uint32_t*)(llr + p.order[b] * p.nsym) = pack4(v[0][b], v[1][b], v[2][b], v[3][b]);
+        }
+        if (!more)
+            break;
+        llr += llr_step;
+        f = fn;
+        a = an;
+        c = cn;
+        n0 = n0n;
     }
 }
 
@@ -305,37 +375,33 @@ struct drx_demapper {
 
 namespace {
 
+template <int BITS>
+cudaError_t launch_bits(const DemapParams& p, dim3 grid, cudaStream_t s)
+{
+    const bool whole = !((uintptr_t)p.sym & 15) && !(p.sym_stride & 3) && !((uintptr_t)p.llr & 7) &&
+                       !(p.llr_stride & 7) && !(p.nsym & 3) && p.nsym * BITS == p.nldpc;
+    if (whole)
+        k_demap_rows<BITS><<<grid, 256, 0, s>>>(p);
+    else
+        k_demap<BITS><<<grid, 256, 0, s>>>(p);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_demap(const DemapParams& p, int sms, cudaStream_t s)
 {
     const int gx = (((p.nsym + 3) / 4) + 255) / 256;
     const int gy = std::max(1, std::min(p.nframes, std::max(1, 8 * sms / gx)));
     const dim3 grid(gx, std::min(gy, 65535));
     switch (p.qpsk ? 2 : p.bits) {
-    case 2:
-        k_demap<2><<<grid, 256, 0, s>>>(p);
-        break;
-    case 3:
-        k_demap<3><<<grid, 256, 0, s>>>(p);
-        break;
-    case 4:
-        k_demap<4><<<grid, 256, 0, s>>>(p);
-        break;
-    case 5:
-        k_demap<5><<<grid, 256, 0, s>>>(p);
-        break;
-    case 6:
-        k_demap<6><<<grid, 256, 0, s>>>(p);
-        break;
-    case 7:
-        k_demap<7><<<grid, 256, 0, s>>>(p);
-        break;
-    case 8:
-        k_demap<8><<<grid, 256, 0, s>>>(p);
-        break;
-    default:
-        return cudaErrorInvalidValue;
+    case 2: return launch_bits<2>(p, grid, s);
+    case 3: return launch_bits<3>(p, grid, s);
+    case 4: return launch_bits<4>(p, grid, s);
+    case 5: return launch_bits<5>(p, grid, s);
+    case 6: return launch_bits<6>(p, grid, s);
+    case 7: return launch_bits<7>(p, grid, s);
+    case 8: return launch_bits<8>(p, grid, s);
     }
-    return cudaGetLastError();
+    return cudaErrorInvalidValue;
 }
 
 }  // namespace
