@@ -32,13 +32,13 @@ namespace drxg {
     X(6, 9, 9, 0, 2) X(7, 12, 12, 0, 2) X(8, 9, 9, 0, 3) X(9, 16, 16, 0, 4) X(10, 20, 20, 0, 3)          \
     X(11, 25, 25, 0, 6) X(12, 28, 28, 0, 4) X(13, 1, 1, 7, 1) X(14, 1, 1, 14, 3) X(15, 1, 1, 22, 5) X(16, 25, 25, 0, 3)
 
-/* One code's frames with its shape: its tables staged in the shape's form,
+/* One code's frames with its shape: its tables staged,
  * then the streaming loop of the frame-pair kernel. */
 template <int A, int B, int GDM, int LS>
 __device__ __noinline__ void mix_code_frames(const DecodeParams& p, const DevCode& c, char* smem, void* msg,
                                              PairLanes& st)
 {
-    const PairFrame fr = stage_pair<false, pair_key_form(A, B, GDM, LS)>(c, smem, nullptr);
+    const PairFrame fr = stage_pair<false>(c, smem, nullptr);
     __syncthreads();
     stream_frames<A, B, GDM, LS, false>(p, c, fr, msg, 0, p.nframes, st);
 }

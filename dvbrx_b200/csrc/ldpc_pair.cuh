@@ -4,17 +4,14 @@
  * they compile in parallel; ldpc_pair.cu holds the host side): the same arithmetic as ldpc_decode.cu
  * (bit-exact to libdvbrx/src/ldpc.c), two frames per CTA.
  *
- * SIMD within a register: every value of the decoder fits 16 bits, so each
- * 32-bit register carries the same quantity for two frames, lane A in the
- * low half and lane B in the high half, and every step of the check node is
- * a native 16x2 instruction on sm_100a (video min/max __vmins2/__vmaxs2,
- * DPX __viaddmax_s16x2 for the saturating add and |x|, the lane-wise __vadd2,
- * PRMT for sign masks and byte packing, an FP16 compare for the message
- * index).  One instruction stream decodes two frames.
+ * SIMD within a register: each 32-bit register carries the same quantity for
+ * two frames as two halves, lane A in the low one and lane B in the high one,
+ * every value of the decoder being exact in one (PairCheck).  One instruction
+ * stream decodes two frames.
  *
  * Shared memory holds both frames' posteriors interleaved: the 16-bit word
- * v holds the int8 posterior of variable v for lane A (low byte) and lane B
- * (high byte): K information bits, then R parity bits in layer order.
+ * v holds the posterior of variable v, plus 128, for lane A (low byte) and
+ * lane B (high byte): K information bits, then R parity bits in layer order.
  *
  * A check node runs on one thread: 360 of the 384 threads hold the 360
  * checks of a layer, every link of a check in registers, no shuffles (two
@@ -24,7 +21,7 @@
  * wavefront levels carry only the links two checks of the layer share.  The
  * thread of a check stores its compressed messages for both frames in one
  * 8-byte record: per lane min0 (6 bits) | min1 << 6 | index << 12, then the
- * sign bits of lane A in the low half and of lane B in the high half.
+ * sign bits.
  *
  * Frames stream through the two lanes independently: when a lane's frame
  * passes the syndrome check or reaches max_iter, its results are written
@@ -59,23 +56,8 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel)
     asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
     return d;
 }
-/* two int8 (low 16 bits) -> int16x2, sign-extended */
-__device__ __forceinline__ uint32_t sx2(uint32_t b) { return prmt(b, 0, 0x9180); }
-/* int16x2 in [-128, 127] -> two bytes (low 16 bits) */
-__device__ __forceinline__ uint32_t pk2(uint32_t v) { return prmt(v, 0, 0x0020); }
 /* 0xFFFF in each lane whose bit 15 is set */
 __device__ __forceinline__ uint32_t lmask(uint32_t v) { return prmt(v, 0, 0xBB99); }
-__device__ __forceinline__ uint32_t sel(uint32_t m, uint32_t a, uint32_t b) { return (m & a) | (~m & b); }
-/* saturating int8 add in int16 lanes */
-__device__ __forceinline__ uint32_t sadd(uint32_t a, uint32_t b)
-{
-    return __vmins2(__viaddmax_s16x2(a, b, 0xFF80FF80u), 0x007F007Fu);
-}
-/* lane-wise |x| = max(~x + 1, x): one LOP3 and one DPX add-max (a 16x2
- * subtract, __vsub2, has no single instruction: it costs three or four) */
-__device__ __forceinline__ uint32_t abs2(uint32_t x) { return __viaddmax_s16x2(~x, 0x00010001u, x); }
-/* lane-wise -x, the 16x2 add (__vadd2) being one instruction */
-__device__ __forceinline__ uint32_t neg2(uint32_t x) { return __vadd2(~x, 0x00010001u); }
 /* 16-bit shared-memory accesses at a 32-bit shared address */
 __device__ __forceinline__ uint32_t lds16(uint32_t a)
 {
@@ -87,11 +69,6 @@ __device__ __forceinline__ void sts16(uint32_t a, uint32_t v)
 {
     asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((unsigned short)v));
 }
-__device__ __forceinline__ uint32_t heq(uint32_t a, uint32_t b)
-{
-    return __heq2_mask(*(const __half2*)&a, *(const __half2*)&b);
-}
-
 /*
  * One check node (i, j) for both lanes, on one thread: link slots
  * k = 0 .. S-1.  Slot 0 is the parity bit, slot 1 the previous parity bit
@@ -100,21 +77,16 @@ __device__ __forceinline__ uint32_t heq(uint32_t a, uint32_t b)
  * value).  The node state lives in registers across the phases of its layer
  * (see layer_pair).  Slot masks and the message index keep slot k at bit k.
  *
- * Minimums are taken over keys |x| * 32 + k (|x| <= 128, so a key fits 13
- * bits of a 16-bit lane): the smallest key gives min0 and the slot holding
- * it, the second smallest min1 (a tie between two slots at min0 puts min1 =
- * min0, and then which slot holds min0 changes no message).  The full
- * passes run every slot without branches: a slot that is not a link, or
- * whose bit an earlier check of the layer writes (read later, in its level),
- * enters the minimums with a key above every real one; stores are
+ * The full passes run every slot without branches: a slot that is not a link,
+ * or whose bit another check of the layer shares (taken in after the layer's
+ * levels), enters the minimums above every real magnitude; stores are
  * predicated.
  *
  * Sign bits of a record: the 16 slots of a word in the byte layout
  * byte 0 = lane A even slots, byte 1 = lane A odd slots, byte 2 = lane B
  * even slots, byte 3 = lane B odd slots, slot 2s (2s + 1) at bit 7 - s of
- * its byte; shifted left by s, the word holds the signs of slots 2s and
- * 2s + 1 in the sign bits of its bytes, which one PRMT turns into lane
- * masks.
+ * its byte: one PRMT takes the signs of two slots of both lanes there, and one
+ * shift brings a slot's back to the halves' sign bits.
  */
 /* A check's message record: 8 bytes up to degree 16 (per lane min0, min1
  * and a 4-bit index in one word, 16 sign bits per lane in the other); 16
@@ -122,21 +94,6 @@ __device__ __forceinline__ uint32_t heq(uint32_t a, uint32_t b)
  * the index, 16 bits per lane). */
 template <bool WIDE>
 using PairRec = typename std::conditional<WIDE, uint4, uint2>::type;
-
-/* key of a slot that takes no part in the minimums */
-constexpr uint32_t kKeyOff = 0x1FE01FE0u; /* 255 * 32 in both lanes */
-
-/* the sign bits of slot k (k < 16) of both lanes in a record word */
-__device__ __forceinline__ constexpr uint32_t sign_bits(int k)
-{
-    return (k & 1) ? (1u << (15 - (k >> 1))) | (1u << (31 - (k >> 1)))
-                   : (1u << (7 - (k >> 1))) | (1u << (23 - (k >> 1)));
-}
-/* lane masks of slot k's sign bits in record word w (k < 16) */
-__device__ __forceinline__ uint32_t sign_mask(uint32_t w, int k)
-{
-    return prmt(w << (k >> 1), 0, (k & 1) ? 0xBB99u : 0xAA88u);
-}
 
 /* The learned magnitudes of the current iteration (learned kernels): byte
  * 1024 h + 128 k + m = min(learned_mag(m, word of lane h's row and degree
@@ -153,28 +110,93 @@ __device__ __forceinline__ uint32_t learned_lut(uint32_t c, uint32_t t)
     return (uint32_t)s_learn_lut[t + (c & 0xFFFFu)] | (uint32_t)s_learn_lut[t + 1024u + (c >> 16)] << 16;
 }
 
-/* WIDE: the kernel's records are 16 bytes (its degree bound is above 16).
- * PO: the parity posteriors (slots 0 and 1) are not in shared memory; the
- * layer loop hands their two-byte words in and takes the new ones back. */
+/*
+ * Values are halves in units of 1/256, exact: a posterior P is kept as the byte
+ * u = P + 128, which one PRMT makes the half 1024 + u, and
+ *     x = sat((1024 + u)/256 - (4 + m)) - 1/2 = (P - m)/256,
+ * the saturating fused multiply-add being the clamp at -128 and one minimum
+ * the clamp at 127 (255/256 before the half is taken off).  |x| is an operand
+ * modifier of the minimum, a link's message magnitude is a fused multiply-add
+ * of the comparison's 1.0, min0 + f (min1 - min0), its sign one LOP3.  The
+ * record's index is a slot that holds min0 (a tie makes min1 = min0, and then
+ * which one changes no message), collected by a fused multiply-add per slot in
+ * chains of about seven.
+ *
+ * Bound by the integer pipe and by issue: the decoder on 16-bit integers had 22
+ * to 28 instructions of the integer pipe per link (minimums, selects, permutes
+ * and both adds; the pipe 76 to 86 % busy with the other pipes idle), this form
+ * about 13, its adds and selects on the other pipe.  us of the GPU per
+ * frame-iteration before and after: S2X 18/30 0.305 and 0.206, normal 2/3 0.297
+ * and 0.279, 8/9 0.264 and 0.223, 9/10 0.331 and 0.257, short 1/2 0.086 and
+ * 0.072, 3/5 0.143 and 0.117; normal 3/5 8PSK, 4096 frames over its waterfall
+ * 37.4 and 31.3 ms.  Measured and not kept: link addresses two in a register or
+ * formed again where 80 registers spill (short 5/6 and 8/9, normal 4/5; fewer
+ * spills, 8 to 25 % slower), one CTA per SM for those.
+ */
+__device__ __forceinline__ __half2 h2(uint32_t a) { return *(const __half2*)&a; }
+__device__ __forceinline__ uint32_t u2(__half2 a) { return *(const uint32_t*)&a; }
+constexpr uint32_t kHUnit = 0x1C001C00u;   /* 1/256 */
+constexpr uint32_t kH127 = 0x37F037F0u;    /* 127/256 */
+constexpr uint32_t kH255 = 0x3BF83BF8u;    /* 255/256 */
+constexpr uint32_t kHHalf = 0x38003800u;   /* 1/2 */
+constexpr uint32_t kH31 = 0x2FC02FC0u;     /* 31/256 */
+constexpr uint32_t kH32 = 0x30003000u;     /* 32/256 */
+constexpr uint32_t kHFour = 0x44004400u;   /* 4 */
+constexpr uint32_t kH256 = 0x5C005C00u;    /* 256 */
+constexpr uint32_t kH1024 = 0x64006400u;   /* 1024: its low bits hold an integer below 1024 */
+constexpr uint32_t kHOne = 0x3C003C00u;    /* above every magnitude */
+constexpr uint32_t kHSign = 0x80008000u;
+constexpr uint32_t kHNegUnit = 0x9C009C00u; /* -1/256 */
+
+/* integers below 1024 in both lanes as halves in 1/256, and back */
+__device__ __forceinline__ uint32_t h_of_int(uint32_t v)
+{
+    return u2(__hfma2(h2(v | kH1024), h2(kHUnit), h2(kHFour | kHSign)));
+}
+__device__ __forceinline__ uint32_t h_to_int(uint32_t v)
+{
+    return u2(__hfma2(h2(v), h2(kH256), h2(kH1024))) & 0x03FF03FFu;
+}
+/* x from a posterior word (two bytes u) and minus 4 minus the message */
+__device__ __forceinline__ uint32_t h_input(uint32_t raw, uint32_t cm)
+{
+    const uint32_t z = u2(__hfma2_sat(h2(prmt(raw, 0x64646464u, 0x4140)), h2(kHUnit), h2(cm)));
+    return u2(__hsub2(__hmin2(h2(z), h2(kH255)), h2(kHHalf)));
+}
+/* the new posterior's two bytes from x and the message */
+__device__ __forceinline__ uint32_t h_output(uint32_t x, uint32_t m)
+{
+    const __half2 z = __hadd2_sat(h2(x), __hadd2(h2(m), h2(kHHalf)));
+    const uint32_t q = u2(__hfma2(__hmin2(z, h2(kH255)), h2(kH256), h2(kH1024)));
+    return prmt(q, 0, 0x0020);
+}
+__device__ __forceinline__ uint32_t h_abs(uint32_t x) { return u2(__habs2(h2(x))); }
+__device__ __forceinline__ uint32_t h_min(uint32_t a, uint32_t b) { return u2(__hmin2(h2(a), h2(b))); }
+__device__ __forceinline__ uint32_t h_max(uint32_t a, uint32_t b) { return u2(__hmax2(h2(a), h2(b))); }
+/* 1.0 in the lanes where a = b */
+__device__ __forceinline__ __half2 h_eq(uint32_t a, uint32_t b) { return __heq2(h2(a), h2(b)); }
+/* max(a - 1/256, 0): the offset */
+__device__ __forceinline__ uint32_t h_offset(uint32_t a)
+{
+    return u2(__hfma2_relu(h2(a), h2(kHOne), h2(kHNegUnit)));
+}
+/* learned magnitudes of capped minimums c */
+__device__ __forceinline__ uint32_t h_learned(uint32_t c, uint32_t lp) { return h_of_int(learned_lut(h_to_int(c), lp)); }
+
 template <int DM, bool EXACT, int LS, bool WIDE, bool PO>
-struct PairCheckKey {
+struct PairCheck {
     static_assert(DM <= (WIDE ? 32 : 16), "degree above the record's slots");
     using Rec = PairRec<WIDE>;
-    static constexpr bool kKeys = true;
     static constexpr int S = DM;
-    /* slots that can be late or early: K0 .. K1 (link slots 2 .. 2 LS + 1) */
     static constexpr int K0 = 2;
     static constexpr int K1 = S - 1 < 2 * LS + 1 ? S - 1 : 2 * LS + 1;
-    uint32_t addr[S]; /* shared-memory byte addresses of the owned links' posteriors */
+    uint32_t addr[S]; /* shared-memory byte addresses of the links' posteriors */
     uint32_t x[S];
-    uint32_t live, inm, outm; /* bit k: slot k is a link / is read late / is written early */
-    uint32_t n0, n1, p0, p1, idxh, sgn, sgn1; /* old messages; sgn: sign bits of slots 0-15, sgn1: 16-31 */
-    uint32_t min0, min1, sg;                  /* smallest keys, sign parity (bit 15 / 31) */
-    uint32_t a0, a1, b0, b1, nidx;            /* outgoing message candidates (set by finish), index */
-    uint32_t recw;                            /* the record's magnitude word (set by finish) */
+    uint32_t live, inm, outm;
+    uint32_t om0, omd, idxh, sgn, sgn1; /* old messages: min0, min1 - min0, index, sign bits */
+    uint32_t min0, min1, sg;            /* smallest magnitudes, sign parity (bit 15 / 31) */
+    uint32_t mn0, mnd, recw;            /* outgoing magnitudes with the parity's sign (set by finish), record word */
 
-    /* ent: the layer's entries (shared byte address of the link group's first
-     * posterior word, -2a), cnt of them */
     __device__ __forceinline__ void setup(const int2* __restrict__ ent, int cnt, int K, int q, int i, int j,
                                           Rec rec, uint32_t fresh, unsigned long long meta, uint32_t sbase)
     {
@@ -196,7 +218,7 @@ struct PairCheckKey {
                 /* a slot past the degree takes the last link's address: read, never used.
                  * Link of check j: word (j - a) mod 360 of the group, as min(u, u + 720)
                  * over unsigned byte offsets u = 2 j - 2 a */
-                const int2 e = ent[min(k, D - 1) - 2];
+                const int2 e = ent[(EXACT ? k : min(k, D - 1)) - 2];
                 const uint32_t u = tj + (uint32_t)e.y;
                 addr[k] = (uint32_t)e.x + __viaddmin_u32(u, 2u * kQCp, u);
             }
@@ -204,98 +226,70 @@ struct PairCheckKey {
         /* messages: zero for a lane in its first iteration */
         const uint32_t w0 = rec.x & ~fresh;
         sgn = rec.y & ~fresh;
-        const uint32_t m0 = w0 & 0x003F003Fu, m1 = (w0 >> 6) & 0x003F003Fu;
         if constexpr (WIDE) {
             sgn1 = rec.z & ~fresh;
-            idxh = (rec.w & ~fresh) | 0x64006400u; /* FP16 1024 + index */
+            idxh = (rec.w & ~fresh) | kH1024;
         } else {
             sgn1 = 0;
-            idxh = ((w0 >> 12) & 0x000F000Fu) | 0x64006400u; /* FP16 1024 + index */
+            idxh = ((w0 >> 12) & 0x000F000Fu) | kH1024;
         }
-        /* minus the message: +m if it is negative, else -min(m, 31) */
-        n0 = m0;
-        n1 = m1;
-        p0 = __viaddmax_s16x2(~m0, 0x00010001u, 0xFFE1FFE1u); /* max(-m, -31) */
-        p1 = __viaddmax_s16x2(~m1, 0x00010001u, 0xFFE1FFE1u);
-        min0 = min1 = kKeyOff;
+        om0 = h_of_int(w0 & 0x003F003Fu);
+        omd = u2(__hsub2(h2(h_of_int((w0 >> 6) & 0x003F003Fu)), h2(om0)));
+        min0 = min1 = kHOne;
         sg = 0;
     }
 
-    /* minus the old message of slot k */
+    /* minus 4 minus the old message of slot k: its magnitude with its sign, at most 31 */
     __device__ __forceinline__ uint32_t unmsg(int k) const
     {
-        const uint32_t im = heq(idxh, 0x64006400u + (uint32_t)k * 0x00010001u);
-        const uint32_t sm = sign_mask(k < 16 ? sgn : sgn1, k & 15);
-        return sel(sm, sel(im, n1, n0), sel(im, p1, p0));
+        const uint32_t mag = u2(__hfma2(h_eq(idxh, kH1024 + (uint32_t)k * 0x00010001u), h2(omd), h2(om0)));
+        const int s = (k & 15) >> 1;
+        const uint32_t m = ((((k < 16 ? sgn : sgn1) << ((k & 1) ? s : s + 8)) & kHSign) ^ mag);
+        return u2(__hsub2(h2(kHFour | kHSign), __hmin2(h2(m), h2(kH31))));
     }
 
-    /* the key of value v in slot k */
-    static __device__ __forceinline__ uint32_t key(uint32_t v, int k)
+    __device__ __forceinline__ void fold(uint32_t a)
     {
-        return abs2(v) * 32u + (uint32_t)k * 0x00010001u;
+        min1 = h_min(min1, h_max(min0, a));
+        min0 = h_min(min0, a);
     }
 
-    __device__ __forceinline__ void fold(uint32_t kv)
-    {
-        min1 = __vmins2(min1, __vmaxs2(min0, kv));
-        min0 = __vmins2(min0, kv);
-    }
-
-    /* every slot but the late ones, without branches; minimums folded
-     * two slots at a time: min1 = second smallest of {min0, min1, a, b} =
-     * min3(max(min0, min(a, b)), min1, max(a, b)).  LEV: the layer has late
-     * slots; otherwise only the slots that can be absent are masked (the
-     * previous parity of check (0, 0)). */
     template <bool LEV>
     __device__ __forceinline__ void read_all(const uint16_t* __restrict__ post, uint32_t r0, uint32_t r1)
     {
-        const uint32_t excl = LEV ? (~live | inm | outm) : ~live;
-        /* slot k read: its value kept in x[k] (minus its old message for a
-         * late slot), its key returned */
+        const uint32_t shared = inm | outm;
         auto slot = [&](int k) {
             const uint32_t m = unmsg(k);
             const uint32_t raw = PO && k < 2 ? (k == 0 ? r0 : r1) : lds16(addr[k]);
-            const uint32_t v = sadd(sx2(raw), m);
-            uint32_t kv = key(v, k);
-            /* shared slots are among K0 .. K1; past them only a non-link (inexact kernels) */
+            uint32_t v = h_input(raw, m);
             const bool maybe_shared = LEV && k >= K0 && k <= K1;
-            if (maybe_shared || !EXACT || k == 1) {
-                /* excluded: not a link, or shared (its sign and key are taken in fold_shared) */
-                const bool ex = (excl >> k) & 1u;
-                kv = ex ? kKeyOff : kv;
-                sg ^= ex ? 0u : v;
-            } else {
-                sg ^= v;
+            if (!EXACT || k == 1) { /* a slot that can be absent: above every minimum, positive */
+                v = ((live >> k) & 1u) ? v : kHOne;
             }
-            if (maybe_shared)
-                x[k] = ((inm >> k) & 1u) ? m : v;
-            else
-                x[k] = v;
-            return kv;
+            x[k] = maybe_shared && ((inm >> k) & 1u) ? m : v; /* a late slot waits for its level */
+            const bool out = maybe_shared && ((shared >> k) & 1u);
+            sg ^= out ? 0u : v;
+            return out ? kHOne : v;
         };
 #pragma unroll
         for (int k = 0; k + 1 < S; k += 2) {
-            const uint32_t a = slot(k), b = slot(k + 1);
-            const uint32_t lo = __vmins2(a, b), hi = __vmaxs2(a, b);
-            min1 = __vimin3_s16x2(__vmaxs2(min0, lo), min1, hi);
-            min0 = __vimin3_s16x2(min0, a, b);
+            const uint32_t a = h_abs(slot(k)), b = h_abs(slot(k + 1));
+            const uint32_t lo = h_min(a, b), hi = h_max(a, b);
+            min1 = __vimin3_s16x2(h_max(min0, lo), min1, hi); /* halves that are not negative order as integers */
+            min0 = h_min(min0, lo);
         }
         if (S & 1)
-            fold(slot(S - 1));
+            fold(h_abs(slot(S - 1)));
     }
 
-    /* the smallest magnitude so far */
-    __device__ __forceinline__ uint32_t smallest() const { return (min0 >> 5) & 0x07FF07FFu; }
+    __device__ __forceinline__ uint32_t smallest() const { return min0; }
 
-    /* a shared slot into the minimums and the sign (use: it is one) */
     __device__ __forceinline__ void fold_shared(int k, bool use)
     {
-        fold(use ? key(x[k], k) : kKeyOff);
+        fold(use ? h_abs(x[k]) : kHOne);
         sg ^= use ? x[k] : 0u;
     }
 
-    /* a thread that holds no check (t >= 360): valid addresses, no links, so
-     * that it can run the warp-uniform level steps of its warp */
     __device__ __forceinline__ void idle(uint32_t sbase)
     {
 #pragma unroll
@@ -304,76 +298,58 @@ struct PairCheckKey {
             x[k] = 0;
         }
         live = inm = outm = 0;
-        n0 = n1 = p0 = p1 = sgn = sgn1 = 0;
-        idxh = 0x64006400u;
-        min0 = min1 = kKeyOff;
-        sg = a0 = a1 = b0 = b1 = nidx = recw = 0;
+        om0 = omd = sgn = sgn1 = 0;
+        idxh = kH1024;
+        min0 = min1 = kHOne;
+        sg = mn0 = mnd = recw = 0;
     }
 
-    /* the cap at 127 and offset 1, or the learned magnitudes of each lane's
-     * iteration (lpA: the check's class table, learned_lut); the
-     * outgoing candidates +-mn0, +-mn1 with the check's sign parity applied
-     * (a0, a1 for a slot whose value is positive, b0 = -a0, b1 = -a1
-     * otherwise) and the record's magnitudes.
-     */
-    __device__ __forceinline__ void finish(bool learned, uint32_t lpA)
+    __device__ __forceinline__ void finish(bool learned, uint32_t lp)
     {
-        const uint32_t c0 = __vmins2((min0 >> 5) & 0x07FF07FFu, 0x007F007Fu);
-        const uint32_t c1 = __vmins2((min1 >> 5) & 0x07FF07FFu, 0x007F007Fu);
-        uint32_t m0, m1;
-        if (learned) {
-            m0 = learned_lut(c0, lpA);
-            m1 = learned_lut(c1, lpA);
-        } else {
-            m0 = __viaddmax_s16x2(c0, 0xFFFFFFFFu, 0u);
-            m1 = __viaddmax_s16x2(c1, 0xFFFFFFFFu, 0u);
-        }
-        const uint32_t sm = lmask(sg), q0 = neg2(m0), q1 = neg2(m1);
-        a0 = sel(sm, q0, m0);
-        a1 = sel(sm, q1, m1);
-        b0 = sel(sm, m0, q0);
-        b1 = sel(sm, m1, q1);
-        nidx = (min0 & 0x001F001Fu) | 0x64006400u; /* FP16 1024 + slot of min0 */
-        /* per lane min0 (6 bits) | min1 << 6, magnitudes capped at 32 (| index << 12 below degree 17) */
-        recw = __vmins2(m0, 0x00200020u) | (__vmins2(m1, 0x00200020u) << 6);
-        if (!WIDE)
-            recw |= (min0 & 0x000F000Fu) << 12;
+        const uint32_t c0 = h_min(min0, kH127), c1 = h_min(min1, kH127);
+        const uint32_t m0 = learned ? h_learned(c0, lp) : h_offset(c0);
+        const uint32_t m1 = learned ? h_learned(c1, lp) : h_offset(c1);
+        mn0 = m0 ^ (sg & kHSign);
+        mnd = u2(__hsub2(h2(m1), h2(m0))) ^ (sg & kHSign);
+        /* per lane min0 (6 bits) | min1 << 6, magnitudes capped at 32 */
+        recw = h_to_int(h_min(m0, kH32)) | (h_to_int(h_min(m1, kH32)) << 6);
     }
 
-    /* new posterior of slot k (two bytes) and the lane mask of its value's sign */
-    __device__ __forceinline__ uint32_t update(int k, uint32_t& xm) const
-    {
-        const uint32_t v = x[k];
-        xm = lmask(v);
-        const uint32_t eq = heq(nidx, 0x64006400u + (uint32_t)k * 0x00010001u);
-        const uint32_t o = sel(xm, sel(eq, b1, b0), sel(eq, a1, a0));
-        return pk2(sadd(v, o));
-    }
-
-    /* every other posterior (predicated stores) and the node's compressed
-     * messages for both lanes: the slot holding min0 and one sign bit per
-     * slot (the outgoing message's: the value's sign times the parity).
-     * PO: the parity words go to o0 and o1. */
     __device__ __forceinline__ void write_rest(uint16_t* __restrict__ post, Rec* __restrict__ dst, uint32_t& o0,
                                                uint32_t& o1)
     {
         const uint32_t wm = live & ~outm;
         uint32_t nsg = 0, nsg1 = 0;
+        /* the index in chains of about seven slots, the highest found */
+        constexpr int CH = (S + 6) / 7;
+        __half2 idxs[CH];
+#pragma unroll
+        for (int q = 0; q < CH; q++)
+            idxs[q] = h2(kH1024);
 #pragma unroll
         for (int k = 0; k < S; k++) {
-            uint32_t xm;
-            const uint32_t nv = update(k, xm);
+            const __half2 f = h_eq(h_abs(x[k]), min0);
+            const uint32_t m = u2(__hfma2(f, h2(mnd), h2(mn0))) ^ (x[k] & kHSign);
+            const uint32_t nv = h_output(x[k], m);
+            __half2& idx = idxs[k % CH];
+            idx = __hfma2(f, __hsub2(h2(kH1024 + (uint32_t)k * 0x00010001u), idx), idx);
             if (PO && k < 2)
                 (k == 0 ? o0 : o1) = nv;
             else if (EXACT && k > K1 && k != 1)
                 sts16(addr[k], nv); /* every slot past K1 is a link written here */
             else if ((wm >> k) & 1u)
                 sts16(addr[k], nv);
-            if (k < 16)
-                nsg |= xm & sign_bits(k);
-            else
-                nsg1 |= xm & sign_bits(k - 16);
+            if ((k & 1) || k == S - 1) {
+                /* the signs of two slots in one permute */
+                const int e = k & ~1;
+                const uint32_t p = (k & 1) ? prmt(x[e], x[k], 0xFBD9) : prmt(x[e], 0, 0xFBD9);
+                (k < 16 ? nsg : nsg1) |= p & (0x01010101u << (7 - ((e & 15) >> 1)));
+            }
         }
+        uint32_t nidx = u2(idxs[0]);
+#pragma unroll
+        for (int q = 1; q < CH; q++)
+            nidx = __vmaxs2(nidx, u2(idxs[q]));
         /* the outgoing signs: each value's sign flipped where the parity is odd */
         const uint32_t pm = lmask(sg);
         nsg ^= pm;
@@ -381,228 +357,32 @@ struct PairCheckKey {
             nsg1 ^= pm;
             __stcg(dst, make_uint4(recw, nsg, nsg1, nidx & 0x001F001Fu));
         } else {
-            __stcg(dst, make_uint2(recw, nsg));
+            __stcg(dst, make_uint2(recw | (nidx & 0x000F000Fu) << 12, nsg));
         }
     }
+
+    /* shared links, see level_step */
+    static __device__ __forceinline__ uint32_t none() { return kHOne; }
+    static __device__ __forceinline__ uint32_t value(uint32_t raw, uint32_t m) { return h_input(raw, m); }
+    template <bool LEARNED>
+    static __device__ __forceinline__ uint32_t inner_of(uint32_t smallest)
+    {
+        return h_min(smallest, kH127);
+    }
+    template <bool LEARNED>
+    static __device__ __forceinline__ uint32_t mag(uint32_t v)
+    {
+        return h_abs(v);
+    }
+    template <bool LEARNED>
+    __device__ __forceinline__ uint32_t updated(int k, uint32_t inner, uint32_t others, uint32_t sign, uint32_t lp) const
+    {
+        const uint32_t r = h_min(inner, others);
+        const uint32_t m = LEARNED ? h_learned(r, lp) : h_offset(r);
+        return h_output(x[k], m ^ ((sg ^ sign) & kHSign));
+    }
+    static __device__ __forceinline__ uint32_t smaller(uint32_t a, uint32_t b) { return h_min(a, b); }
 };
-
-/*
- * The previous form of the check node (min form), kept for the kernels where
- * it measures faster (low check degrees, and levelled codes whose wavefront
- * steps wait on the check's finish): minimums over |x| itself, the index of
- * min0 found in the write pass (|x| > min0 per slot), sign bits of slot k
- * at bit k (lane A) and 16 + k (lane B), entries as (shared byte address of
- * the link for check 0 before the wrap, a).  Both forms give the reference's
- * results; a kernel uses one form throughout (its records, entries and
- * syndrome scan).
- */
-template <int DM, bool EXACT, int LS, bool WIDE, bool PO>
-struct PairCheckMin {
-    static_assert(DM <= (WIDE ? 32 : 16), "degree above the record's slots");
-    using Rec = PairRec<WIDE>;
-    static constexpr bool kKeys = false;
-    static constexpr int S = DM;
-    /* slots that can be late or early: K0 .. K1 (link slots 2 .. 2 LS + 1) */
-    static constexpr int K0 = 2;
-    static constexpr int K1 = S - 1 < 2 * LS + 1 ? S - 1 : 2 * LS + 1;
-    uint32_t addr[S]; /* shared-memory byte addresses of the owned links' posteriors */
-    uint32_t x[S];
-    uint32_t live, inm, outm; /* bit k: slot k is a link / is read late / is written early */
-    uint32_t n0, n1, p0, p1, idxh, sgn, sgn1; /* sgn: sign bits of slots 0-15, sgn1: 16-31 */
-    uint32_t min0, min1, sg, mn0, mn1;
-    uint32_t m0p1, nmn0, nmn1; /* min0 + 1, -mn0, -mn1 (set by finish) */
-
-    __device__ __forceinline__ void setup(const int2* __restrict__ ent, int cnt, int K, int q, int i, int j,
-                                          Rec rec, uint32_t fresh, unsigned long long meta, uint32_t sbase)
-    {
-        const int D = EXACT ? DM : cnt + 2;
-        const int pc = K + kQCp * i + j;
-        const int pp = i ? pc - kQCp : K + kQCp * (q - 1) + j - 1;
-        uint32_t lv = (1u << D) - 1u;
-        if ((i | j) == 0)
-            lv &= ~2u;
-        live = lv;
-        inm = (uint32_t)(meta >> 8) & 0xFFFFFFu;
-        outm = (uint32_t)(meta >> 32) & 0xFFFFFFu;
-#pragma unroll
-        for (int k = 0; k < S; k++) {
-            if (k < 2) {
-                addr[k] = PO ? 0u : sbase + 2u * (uint32_t)(k == 0 ? pc : pp);
-            } else {
-                /* a slot past the degree takes the last link's address: read, never used */
-                const int2 e = ent[min(k, D - 1) - 2];
-                addr[k] = (uint32_t)e.x + 2u * (uint32_t)j + (j < e.y ? 2u * kQCp : 0u);
-            }
-        }
-        /* messages: zero for a lane in its first iteration */
-        const uint32_t w0 = rec.x & ~fresh;
-        sgn = rec.y & ~fresh;
-        const uint32_t m0 = w0 & 0x003F003Fu, m1 = (w0 >> 6) & 0x003F003Fu;
-        if constexpr (WIDE) {
-            sgn1 = rec.z & ~fresh;
-            idxh = (rec.w & ~fresh) | 0x64006400u; /* FP16 1024 + index */
-        } else {
-            sgn1 = 0;
-            idxh = ((w0 >> 12) & 0x000F000Fu) | 0x64006400u; /* FP16 1024 + index */
-        }
-        /* minus the message: +m if it is negative, else -min(m, 31) */
-        n0 = m0;
-        n1 = m1;
-        p0 = __viaddmax_s16x2(~m0, 0x00010001u, 0xFFE1FFE1u); /* max(-m, -31) */
-        p1 = __viaddmax_s16x2(~m1, 0x00010001u, 0xFFE1FFE1u);
-        min0 = min1 = 0x00FF00FFu;
-        sg = 0;
-    }
-
-    /* minus the old message of slot k */
-    __device__ __forceinline__ uint32_t unmsg(int k) const
-    {
-        const uint32_t im = heq(idxh, 0x64006400u + (uint32_t)k * 0x00010001u);
-        const uint32_t sm = lmask((k < 16 ? sgn : sgn1) << (15 - (k & 15)));
-        return sel(sm, sel(im, n1, n0), sel(im, p1, p0));
-    }
-
-    __device__ __forceinline__ void fold(uint32_t v)
-    {
-        const uint32_t a = abs2(v);
-        min1 = __vmins2(min1, __vmaxs2(min0, a));
-        min0 = __vmins2(min0, a);
-        sg ^= v;
-    }
-
-    /* every slot but the late ones, without branches; minimums folded
-     * two slots at a time: min1 = second smallest of {min0, min1, a, b} =
-     * min3(max(min0, min(a, b)), min1, max(a, b)).  LEV: the layer has late
-     * slots; otherwise only the slots that can be absent are masked (the
-     * previous parity of check (0, 0)). */
-    template <bool LEV>
-    __device__ __forceinline__ void read_all(const uint16_t* __restrict__ post, uint32_t r0, uint32_t r1)
-    {
-        const uint32_t shared = inm | outm;
-        uint32_t f[S];
-#pragma unroll
-        for (int k = 0; k < S; k++) {
-            const uint32_t m = unmsg(k);
-            const uint32_t raw = PO && k < 2 ? (k == 0 ? r0 : r1) : lds16(addr[k]);
-            uint32_t v = sadd(sx2(raw), m);
-            if (!EXACT || k == 1) /* a slot that can be absent: above every minimum */
-                v = ((live >> k) & 1u) ? v : 0x00FF00FFu;
-            const bool maybe_shared = LEV && k >= K0 && k <= K1;
-            f[k] = maybe_shared && ((shared >> k) & 1u) ? 0x00FF00FFu : v;
-            /* a late slot keeps minus its old message for its level */
-            x[k] = maybe_shared && ((inm >> k) & 1u) ? m : v;
-        }
-#pragma unroll
-        for (int k = 0; k + 1 < S; k += 2) {
-            const uint32_t a = abs2(f[k]), b = abs2(f[k + 1]);
-            const uint32_t lo = __vmins2(a, b), hi = __vmaxs2(a, b);
-            min1 = __vimin3_s16x2(__vmaxs2(min0, lo), min1, hi);
-            min0 = __vimin3_s16x2(min0, a, b);
-            sg ^= f[k] ^ f[k + 1];
-        }
-        if (S & 1)
-            fold(f[S - 1]);
-    }
-
-    /* the smallest magnitude so far */
-    __device__ __forceinline__ uint32_t smallest() const { return min0; }
-
-    /* a shared slot into the minimums and the sign (use: it is one) */
-    __device__ __forceinline__ void fold_shared(int k, bool use) { fold(use ? x[k] : 0x00FF00FFu); }
-
-    /* a thread that holds no check (t >= 360): valid addresses, no links, so
-     * that it can run the warp-uniform level steps of its warp */
-    __device__ __forceinline__ void idle(uint32_t sbase)
-    {
-#pragma unroll
-        for (int k = 0; k < S; k++) {
-            addr[k] = sbase;
-            x[k] = 0x00FF00FFu;
-        }
-        live = inm = outm = 0;
-        n0 = n1 = p0 = p1 = sgn = sgn1 = 0;
-        idxh = 0x64006400u;
-        min0 = min1 = 0x00FF00FFu;
-        sg = mn0 = mn1 = m0p1 = nmn0 = nmn1 = 0;
-    }
-
-    /* the cap at 127 and offset 1, or the learned magnitudes of each lane's
-     * iteration (lpA: the check's class table, learned_lut).
-     */
-    __device__ __forceinline__ void finish(bool learned, uint32_t lpA)
-    {
-        const uint32_t c1 = min1, c0 = min0;
-        uint32_t m0, m1;
-        if (learned) {
-            m0 = learned_lut(__vmins2(c0, 0x007F007Fu), lpA);
-            m1 = learned_lut(__vmins2(c1, 0x007F007Fu), lpA);
-        } else {
-            m0 = __viaddmax_s16x2(__vmins2(c0, 0x007F007Fu), 0xFFFFFFFFu, 0u);
-            m1 = __viaddmax_s16x2(__vmins2(c1, 0x007F007Fu), 0xFFFFFFFFu, 0u);
-        }
-        mn0 = m0;
-        mn1 = m1;
-        m0p1 = __vadd2(c0, 0x00010001u);
-        nmn0 = neg2(m0);
-        nmn1 = neg2(m1);
-    }
-
-    /* new posterior of slot k (two bytes), and its masks: lanes where
-     * |x| is above min0 (the slot does not hold the minimum) and lanes whose
-     * outgoing message is negative */
-    __device__ __forceinline__ uint32_t update(int k, uint32_t& above, uint32_t& neg) const
-    {
-        const uint32_t v = x[k];
-        /* min0 - |x| = min(min0 + x, (min0 + 1) + ~x) < 0 */
-        above = lmask(__viaddmin_s16x2(~v, m0p1, __vadd2(min0, v)));
-        neg = lmask(sg ^ v);
-        const uint32_t o = sel(neg, sel(above, nmn0, nmn1), sel(above, mn0, mn1));
-        return pk2(sadd(v, o));
-    }
-
-    /* every other posterior (predicated stores) and the node's compressed
-     * messages for both lanes, stored by thread 0: the slot holding min0 and
-     * one sign bit per slot.  PO: the parity words go to o0 and o1. */
-    __device__ __forceinline__ void write_rest(uint16_t* __restrict__ post, Rec* __restrict__ dst, uint32_t& o0,
-                                               uint32_t& o1)
-    {
-        const uint32_t wm = live & ~outm;
-        uint32_t nidx = 0, nsg = 0, nsg1 = 0; /* nidx per lane: k + 1 of a slot holding min0, 0 if none */
-#pragma unroll
-        for (int k = 0; k < S; k++) {
-            uint32_t above, neg;
-            const uint32_t nv = update(k, above, neg);
-            if (PO && k < 2)
-                (k == 0 ? o0 : o1) = nv;
-            else if ((wm >> k) & 1u)
-                sts16(addr[k], nv);
-            nidx = sel(above, nidx, (uint32_t)(k + 1) * 0x00010001u);
-            if (k < 16)
-                nsg |= neg & (0x00010001u << k);
-            else
-                nsg1 |= neg & (0x00010001u << (k - 16));
-        }
-        nidx = __viaddmax_s16x2(nidx, 0xFFFFFFFFu, 0u); /* slot number: max(nidx - 1, 0) */
-        const uint32_t m0c = __vmins2(mn0, 0x00200020u), m1c = __vmins2(mn1, 0x00200020u);
-        if constexpr (WIDE)
-            __stcg(dst, make_uint4(m0c | (m1c << 6), nsg, nsg1, nidx));
-        else
-            __stcg(dst, make_uint2(m0c | (m1c << 6) | (nidx << 12), nsg));
-    }
-};
-
-
-/* The form a kernel uses: the key form where it measured faster (normal
- * 1/2 and 3/5, whose layers have 5 and 9 information links and one pair of
- * shared links, and check degrees 22 and above), the min form elsewhere. */
-__host__ __device__ constexpr bool pair_key_form(int a, int b, int gdm, int ls)
-{
-    return gdm == 0 && ((a == b && (a == 5 || a == 9) && ls <= 2) || a >= 20);
-}
-
-template <int DM, bool EXACT, int LS, bool WIDE, bool PO, bool KEYS>
-using PairCheck = typename std::conditional<KEYS, PairCheckKey<DM, EXACT, LS, WIDE, PO>,
-                                            PairCheckMin<DM, EXACT, LS, WIDE, PO>>::type;
 
 struct PairFrame {
     uint16_t* post;
@@ -618,7 +398,7 @@ struct PairFrame {
 
 __device__ __forceinline__ size_t a16p(size_t v) { return (v + 15) & ~(size_t)15; }
 
-template <bool PO, bool KEYS>
+template <bool PO>
 __device__ PairFrame stage_pair(const DevCode& c, char* smem, uint16_t* gpar)
 {
     PairFrame f;
@@ -635,16 +415,13 @@ __device__ PairFrame stage_pair(const DevCode& c, char* smem, uint16_t* gpar)
     uint16_t* eoff = (uint16_t*)(smem + off);
     off += a16p(sizeof(uint16_t) * (c.q + 1));
     uint32_t* steps = (uint32_t*)(smem + off);
-    /* entries (360 g - a, a) as, in the key form, (shared byte address of
-     * group g's first posterior word, -2 a): the link of check j is word
-     * (j - a) mod 360 of the group, at byte offset min(u, u + 720),
-     * u = 2 j - 2 a unsigned; in the min form (shared byte address of the
-     * link of check 0 before the wrap, a): x + 2 j, + 720 if j < a */
+    /* entries (360 g - a, a) as (shared byte address of group g's first
+     * posterior word, -2 a): the link of check j is word (j - a) mod 360 of
+     * the group, at byte offset min(u, u + 720), u = 2 j - 2 a unsigned */
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(f.post);
     for (int k = threadIdx.x; k < c.nent; k += blockDim.x) {
         const int2 e = c.ent[k];
-        ent[k] = KEYS ? make_int2((int)(sbase + 2u * (uint32_t)(e.x + e.y)), -2 * e.y)
-                      : make_int2((int)(sbase + 2u * (uint32_t)e.x), e.y);
+        ent[k] = make_int2((int)(sbase + 2u * (uint32_t)(e.x + e.y)), -2 * e.y);
     }
     for (int k = threadIdx.x; k <= c.q; k += blockDim.x)
         eoff[k] = c.eoff[k];
@@ -665,6 +442,8 @@ __device__ __forceinline__ uint8_t* parity_byte(const DevCode& c, const PairFram
     return ii + 1 < (uint32_t)c.q ? (uint8_t*)fr.gpar + 2 * (kQCp * ii + jj) + h : (uint8_t*)fr.wrap + 2 * jj + h;
 }
 
+constexpr uint32_t kBias = 0x80808080u; /* posterior bytes are P + 128 */
+
 /* Frame f's LLRs into byte `h` of every posterior word (f < 0: the all-zero
  * codeword at full confidence, which passes every check). */
 template <bool PO>
@@ -674,22 +453,26 @@ __device__ void load_lane(const DevCode& c, const PairFrame& fr, const int8_t* _
     const int t = threadIdx.x;
     if (!src) {
         for (int v = t; v < c.K; v += blockDim.x)
-            b[2 * v] = 127;
+            b[2 * v] = 255;
         for (int k = t; k < c.R; k += blockDim.x)
-            *parity_byte<PO>(c, fr, k / kQCp, k % kQCp, h) = 127;
+            *parity_byte<PO>(c, fr, k / kQCp, k % kQCp, h) = 255;
         return;
     }
     if (((uintptr_t)src & 7) == 0) {
         const uint2* s8 = (const uint2*)src;
         for (int u = t; u < c.K / 8; u += blockDim.x) {
-            const uint2 w = __ldcs(s8 + u);
+            uint2 w = __ldcs(s8 + u);
+            w.x ^= kBias;
+            w.y ^= kBias;
 #pragma unroll
             for (int r = 0; r < 8; r++)
                 b[2 * (8 * u + r)] = (uint8_t)((r < 4 ? w.x : w.y) >> (8 * (r & 3)));
         }
         const uint32_t qm = 0xFFFFFFFFu / (uint32_t)c.q + 1u;
         for (int u = t; u < c.R / 8; u += blockDim.x) {
-            const uint2 w = __ldcs(s8 + c.K / 8 + u);
+            uint2 w = __ldcs(s8 + c.K / 8 + u);
+            w.x ^= kBias;
+            w.y ^= kBias;
 #pragma unroll
             for (int r = 0; r < 8; r++) {
                 const uint32_t k = 8u * u + r;
@@ -699,9 +482,9 @@ __device__ void load_lane(const DevCode& c, const PairFrame& fr, const int8_t* _
         }
     } else {
         for (int v = t; v < c.K; v += blockDim.x)
-            b[2 * v] = (uint8_t)src[v];
+            b[2 * v] = (uint8_t)(src[v] ^ 0x80);
         for (int k = t; k < c.R; k += blockDim.x)
-            *parity_byte<PO>(c, fr, k % c.q, k / c.q, h) = (uint8_t)src[c.K + k];
+            *parity_byte<PO>(c, fr, k % c.q, k / c.q, h) = (uint8_t)(src[c.K + k] ^ 0x80);
     }
 }
 
@@ -719,14 +502,14 @@ __device__ __forceinline__ void parity_words(const DevCode& c, const PairFrame& 
 {
     if (PO) {
         pc = i + 1 < c.q ? fr.gpar[kQCp * i + j] : fr.wrap[j];
-        pp = i ? fr.gpar[kQCp * (i - 1) + j] : (j ? fr.wrap[j - 1] : 0x0101u);
+        pp = i ? fr.gpar[kQCp * (i - 1) + j] : (j ? fr.wrap[j - 1] : 0x8181u);
     } else {
         pc = fr.post[c.K + kQCp * i + j];
-        pp = i ? fr.post[c.K + kQCp * (i - 1) + j] : (j ? fr.post[c.K + kQCp * (c.q - 1) + j - 1] : 0x0101u);
+        pp = i ? fr.post[c.K + kQCp * (i - 1) + j] : (j ? fr.post[c.K + kQCp * (c.q - 1) + j - 1] : 0x8181u);
     }
 }
 
-template <bool PO, bool KEYS>
+template <bool PO>
 __device__ int syndrome_pair(const DevCode& c, const PairFrame& fr, volatile int* sflag, volatile int* srow)
 {
     const int t = threadIdx.x;
@@ -755,27 +538,24 @@ __device__ int syndrome_pair(const DevCode& c, const PairFrame& fr, volatile int
                     break;
                 }
                 const int i = row(k);
-                const uint32_t pc = sx2(bc[d]), pp = sx2(bp[d]);
+                const uint32_t pc = bc[d], pp = bp[d];
                 if (k + D * nh < c.q)
                     parity_words<PO>(c, fr, row(k + D * nh), j, bc[d], bp[d]);
-                uint32_t par = pc ^ pp;
-                uint32_t z = (__vadd2(pc, 0xFFFFFFFFu) & ~pc) | (__vadd2(pp, 0xFFFFFFFFu) & ~pp);
-                const int e1 = fr.eoff[i + 1];
-                for (int e = fr.eoff[i]; e < e1; e++) {
+                /* bit 7 of a byte is set for a value that is not negative, and a byte is
+                 * not 0x80 (a value not zero) if its low bits are not zero or bit 7 is clear */
+                auto nonzero = [](uint32_t w) { return ((w & 0x7F7Fu) + 0x7F7Fu) | ~w; };
+                uint32_t par = pc ^ pp, nz = nonzero(pc) & nonzero(pp);
+                const int e0 = fr.eoff[i], e1 = fr.eoff[i + 1];
+                for (int e = e0; e < e1; e++) {
                     const int2 en = fr.ent[e];
-                    uint32_t a;
-                    if (KEYS) {
-                        const uint32_t u = 2u * (uint32_t)j + (uint32_t)en.y;
-                        a = (uint32_t)en.x + __viaddmin_u32(u, 2u * kQCp, u);
-                    } else {
-                        a = (uint32_t)en.x + 2u * (uint32_t)j + (j < en.y ? 2u * kQCp : 0u);
-                    }
-                    const uint32_t v = sx2(lds16(a));
-                    par ^= v;
-                    z |= __vadd2(v, 0xFFFFFFFFu) & ~v;
+                    const uint32_t u = 2u * (uint32_t)j + (uint32_t)en.y;
+                    const uint32_t w = lds16((uint32_t)en.x + __viaddmin_u32(u, 2u * kQCp, u));
+                    par ^= w;
+                    nz &= nonzero(w);
                 }
-                const uint32_t bad = (par | z);
-                const int f = ((bad >> 15) & 1) | ((bad >> 30) & 2);
+                /* the bits that are not set count the negative values: all links less the set ones */
+                const uint32_t bad = (((e1 - e0) & 1) ? ~par : par) | ~nz;
+                const int f = ((bad >> 7) & 1) | ((bad >> 14) & 2);
                 if (f & ~fail) {
                     fail |= f;
                     atomicOr((int*)sflag, f);
@@ -799,20 +579,22 @@ __device__ int syndrome_pair(const DevCode& c, const PairFrame& fr, volatile int
  * before it, so the step is kept to the chain from a late slot's posterior to
  * an early slot's: the message to a shared slot has the magnitude of the
  * smallest other link, min(inner, the other shared slots), where `inner`, the
- * outgoing magnitude of the links no other check of the layer shares, is
- * known before the first level, and the sign of the others' signs.  The
+ * smallest of the links no other check of the layer shares, capped, is known
+ * before the first level, and the sign of the others' signs.  The
  * node's minimums take the shared slots after the last level (fold_shared).
  * Shared links come first in every layer (codes.cpp), so they are among slots
- * 2 .. KE: two for KE = 3, three or four for KE = 5.
- * lp: the check's learned class table (learned kernels; inner is then the
- * capped minimum itself).
+ * 2 .. KE: two for KE = 3, three or four for KE = 5, and so on.
+ * lp: the check's learned class table (learned kernels).
  *
  * Bound by that chain's latency, 3 to 4 warps a level between CTA barriers: it
  * took the node's whole finish (minimums, both candidates, the index) and every
  * shared slot's update before.  With two, four, six and more slots compiled
  * apart, us of the GPU per frame-iteration: normal 3/5 0.400 -> 0.376, 1/3
  * 0.426 -> 0.378, 5/6 0.407 -> 0.340, 8/9 0.360 -> 0.264, short 1/2 0.095 ->
- * 0.086, 3/5 0.181 -> 0.143, 5/6 0.182 -> 0.157.
+ * 0.086, 3/5 0.181 -> 0.143, 5/6 0.182 -> 0.157 (all with the node on 16-bit
+ * integers).  The forms are written out: one form over every slot's test that
+ * takes the two smallest left normal 9/10 at 0.342 and 4/5 at 0.294, which run
+ * at 0.257 and 0.249.
  */
 template <int KE, class Ck>
 __device__ __forceinline__ void read_late(Ck& ck, bool mine)
@@ -820,7 +602,7 @@ __device__ __forceinline__ void read_late(Ck& ck, bool mine)
     const uint32_t im = mine ? ck.inm : 0u;
 #pragma unroll
     for (int k = Ck::K0; k <= KE; k++) {
-        const uint32_t v = sadd(sx2(lds16(ck.addr[k])), ck.x[k]);
+        const uint32_t v = Ck::value(lds16(ck.addr[k]), ck.x[k]);
         ck.x[k] = (im >> k) & 1u ? v : ck.x[k];
     }
 }
@@ -828,28 +610,24 @@ __device__ __forceinline__ void read_late(Ck& ck, bool mine)
 template <int KE, bool LEARNED, class Ck>
 __device__ __forceinline__ void level_step(Ck& ck, uint32_t inner, bool mine, bool late, uint32_t lp)
 {
-    constexpr uint32_t NONE = 0x00FF00FFu; /* above every magnitude */
+    const uint32_t NONE = Ck::none(); /* above every magnitude */
     const uint32_t im = mine ? ck.inm : 0u, om = mine ? ck.outm : 0u, sh = ck.inm | ck.outm;
-    /* max(|x| - 1, 0), by -x - 1 = ~x; |x| in learned kernels */
-    auto mag = [](uint32_t v) { return LEARNED ? abs2(v) : __viaddmax_s16x2_relu(v, 0xFFFFFFFFu, ~v); };
     auto read = [&](int k) {
         if (late) {
-            const uint32_t v = sadd(sx2(lds16(ck.addr[k])), ck.x[k]);
+            const uint32_t v = Ck::value(lds16(ck.addr[k]), ck.x[k]);
             ck.x[k] = (im >> k) & 1u ? v : ck.x[k];
         }
-        return mag(ck.x[k]);
+        return Ck::template mag<LEARNED>(ck.x[k]);
     };
     /* slot k, the smallest magnitude and the sign of the other shared slots */
     auto write = [&](int k, uint32_t others, uint32_t sign) {
-        const uint32_t v = ck.x[k], r = __vmins2(inner, others);
-        const uint32_t m = LEARNED ? learned_lut(r, lp) : r;
-        /* both signs side by side: v - m = (v + 1) + ~m */
-        const uint32_t up = sadd(v, m), down = sadd(__vadd2(v, 0x00010001u), ~m);
-        const uint32_t nv = pk2(sel(lmask(ck.sg ^ sign), down, up));
+        const uint32_t nv = ck.template updated<LEARNED>(k, inner, others, sign, lp);
         if ((om >> k) & 1u)
             sts16(ck.addr[k], nv);
     };
-    if constexpr (KE == 3) {
+    if constexpr (KE < 3) {
+        return; /* no two links of a layer are shared */
+    } else if constexpr (KE == 3) {
         const uint32_t a = read(2), b = read(3);
         write(2, b, ck.x[3]);
         write(3, a, ck.x[2]);
@@ -857,26 +635,86 @@ __device__ __forceinline__ void level_step(Ck& ck, uint32_t inner, bool mine, bo
         const bool four = (sh >> 5) & 1u;
         const uint32_t a = read(2), b = read(3), c = read(4), r5 = read(5);
         const uint32_t d = four ? r5 : NONE;
-        const uint32_t ab = __vmins2(a, b), cd = __vmins2(c, d);
+        const uint32_t ab = Ck::smaller(a, b), cd = Ck::smaller(c, d);
         const uint32_t sab = ck.x[2] ^ ck.x[3], s5 = four ? ck.x[5] : 0u, scd = ck.x[4] ^ s5;
-        write(2, __vmins2(b, cd), ck.x[3] ^ scd);
-        write(3, __vmins2(a, cd), ck.x[2] ^ scd);
-        write(4, __vmins2(ab, d), sab ^ s5);
-        write(5, __vmins2(ab, c), sab ^ ck.x[4]);
-    } else {
-        /* the two smallest: a slot that holds the smallest takes the second */
-        uint32_t m0 = NONE, m1 = NONE, sign = 0;
+        write(2, Ck::smaller(b, cd), ck.x[3] ^ scd);
+        write(3, Ck::smaller(a, cd), ck.x[2] ^ scd);
+        write(4, Ck::smaller(ab, d), sab ^ s5);
+        write(5, Ck::smaller(ab, c), sab ^ ck.x[4]);
+    } else if constexpr (KE == 7) { /* five or six */
+        const bool six = (sh >> 7) & 1u;
+        const uint32_t a = read(2), b = read(3), c = read(4), d = read(5), e = read(6), r7 = read(7);
+        const uint32_t f = six ? r7 : NONE;
+        const uint32_t ab = Ck::smaller(a, b), cd = Ck::smaller(c, d), ef = Ck::smaller(e, f);
+        const uint32_t abcd = Ck::smaller(ab, cd), abef = Ck::smaller(ab, ef), cdef = Ck::smaller(cd, ef);
+        const uint32_t sab = ck.x[2] ^ ck.x[3], scd = ck.x[4] ^ ck.x[5], s7 = six ? ck.x[7] : 0u, sef = ck.x[6] ^ s7;
+        write(2, Ck::smaller(b, cdef), ck.x[3] ^ scd ^ sef);
+        write(3, Ck::smaller(a, cdef), ck.x[2] ^ scd ^ sef);
+        write(4, Ck::smaller(d, abef), ck.x[5] ^ sab ^ sef);
+        write(5, Ck::smaller(c, abef), ck.x[4] ^ sab ^ sef);
+        write(6, Ck::smaller(f, abcd), s7 ^ sab ^ scd);
+        write(7, Ck::smaller(e, abcd), ck.x[6] ^ sab ^ scd);
+    } else if constexpr (KE == 9) { /* seven or eight */
+        const bool eight = (sh >> 9) & 1u;
+        const uint32_t a = read(2), b = read(3), c = read(4), d = read(5), e = read(6), f = read(7), g = read(8),
+                       r9 = read(9);
+        const uint32_t h = eight ? r9 : NONE;
+        const uint32_t ab = Ck::smaller(a, b), cd = Ck::smaller(c, d), ef = Ck::smaller(e, f), gh = Ck::smaller(g, h);
+        const uint32_t abcd = Ck::smaller(ab, cd), efgh = Ck::smaller(ef, gh);
+        const uint32_t s9 = eight ? ck.x[9] : 0u, s25 = ck.x[2] ^ ck.x[3] ^ ck.x[4] ^ ck.x[5],
+                       s69 = ck.x[6] ^ ck.x[7] ^ ck.x[8] ^ s9, all = s25 ^ s69;
+        uint32_t rest = Ck::smaller(cd, efgh);
+        write(2, Ck::smaller(b, rest), all ^ ck.x[2]);
+        write(3, Ck::smaller(a, rest), all ^ ck.x[3]);
+        rest = Ck::smaller(ab, efgh);
+        write(4, Ck::smaller(d, rest), all ^ ck.x[4]);
+        write(5, Ck::smaller(c, rest), all ^ ck.x[5]);
+        rest = Ck::smaller(gh, abcd);
+        write(6, Ck::smaller(f, rest), all ^ ck.x[6]);
+        write(7, Ck::smaller(e, rest), all ^ ck.x[7]);
+        rest = Ck::smaller(ef, abcd);
+        write(8, Ck::smaller(h, rest), all ^ ck.x[8]);
+        write(9, Ck::smaller(g, rest), all ^ ck.x[9]);
+    } else { /* nine to twelve (or, in a kernel without the forms above, fewer) */
+        uint32_t r[12], sx[12];
 #pragma unroll
-        for (int k = Ck::K0; k <= KE; k++) {
-            const bool is = (sh >> k) & 1u;
-            const uint32_t r = read(k), g = is ? r : NONE;
-            m1 = __vmins2(m1, __vmaxs2(m0, g));
-            m0 = __vmins2(m0, g);
-            sign ^= is ? ck.x[k] : 0u;
+        for (int n = 0; n < 12; n++) {
+            const int k = 2 + n;
+            r[n] = NONE;
+            sx[n] = 0;
+            if (k <= KE) {
+                const bool is = n < 5 || ((sh >> k) & 1u);
+                const uint32_t v = read(k);
+                r[n] = is ? v : NONE;
+                sx[n] = is ? ck.x[k] : 0u;
+            }
         }
-#pragma unroll
-        for (int k = Ck::K0; k <= KE; k++)
-            write(k, sel(heq(mag(ck.x[k]), m0), m1, m0), sign ^ ck.x[k]);
+        constexpr bool MORE = KE > 9;
+        const uint32_t ab = Ck::smaller(r[0], r[1]), cd = Ck::smaller(r[2], r[3]), ef = Ck::smaller(r[4], r[5]),
+                       gh = Ck::smaller(r[6], r[7]);
+        const uint32_t ij = MORE ? Ck::smaller(r[8], r[9]) : NONE, kl = MORE ? Ck::smaller(r[10], r[11]) : NONE;
+        const uint32_t ijkl = MORE ? Ck::smaller(ij, kl) : NONE;
+        auto with = [&](uint32_t v) { return MORE ? Ck::smaller(v, ijkl) : v; };
+        const uint32_t abcd = Ck::smaller(ab, cd), efgh = Ck::smaller(ef, gh);
+        const uint32_t lo = with(efgh), hi = with(abcd);
+        uint32_t all = sx[0] ^ sx[1] ^ sx[2] ^ sx[3] ^ sx[4] ^ sx[5] ^ sx[6] ^ sx[7];
+        if (MORE)
+            all ^= sx[8] ^ sx[9] ^ sx[10] ^ sx[11];
+        auto pair = [&](int n, uint32_t rest) { /* rest: the other pairs */
+            if (2 + n <= KE)
+                write(2 + n, Ck::smaller(r[n + 1], rest), all ^ ck.x[2 + n]);
+            if (3 + n <= KE)
+                write(3 + n, Ck::smaller(r[n], rest), all ^ ck.x[3 + n]);
+        };
+        pair(0, Ck::smaller(cd, lo));
+        pair(2, Ck::smaller(ab, lo));
+        pair(4, Ck::smaller(gh, hi));
+        pair(6, Ck::smaller(ef, hi));
+        if constexpr (MORE) {
+            const uint32_t all8 = Ck::smaller(abcd, efgh);
+            pair(8, Ck::smaller(kl, all8));
+            pair(10, Ck::smaller(ij, all8));
+        }
     }
 }
 
@@ -891,7 +729,7 @@ __device__ __forceinline__ void level_step(Ck& ck, uint32_t inner, bool mine, bo
  * layer share, so the wavefront levels carry just those links.  Unlevelled
  * layers take one pass.
  */
-template <int DM, bool EXACT, int LS, bool WIDE, bool LEARNED, bool PO, bool KEYS>
+template <int DM, bool EXACT, int LS, bool WIDE, bool LEARNED, bool PO>
 __device__ __forceinline__ void layer_pair(const PairFrame& fr, const DevCode& c, int i, int cnt, int nlev,
                                            PairRec<WIDE> rec, unsigned long long meta, uint32_t fresh,
                                            PairRec<WIDE>* __restrict__ msg, int lA, int lB, uint32_t r0,
@@ -904,7 +742,7 @@ __device__ __forceinline__ void layer_pair(const PairFrame& fr, const DevCode& c
     auto lclass = [&]() {
         return LEARNED ? 128u * (uint32_t)s_learn_cls[(EXACT ? DM : cnt + 2) - ((i | j) == 0)] : 0u;
     };
-    using Ck = PairCheck<DM, EXACT, LS, WIDE, PO, KEYS>;
+    using Ck = PairCheck<DM, EXACT, LS, WIDE, PO>;
     Ck ck;
     if (active) {
         ck.setup(fr.ent + fr.eoff[i], cnt, c.K, c.q, i, j, rec, fresh, meta,
@@ -925,8 +763,7 @@ __device__ __forceinline__ void layer_pair(const PairFrame& fr, const DevCode& c
          * last slot that can be late or early in this warp (most
          * layers share one pair of links: link slots 2 and 3 only) */
         const int lev = active ? (int)(meta & 0xFF) : -1;
-        const uint32_t cap = __vmins2(ck.smallest(), 0x007F007Fu);
-        const uint32_t inner = LEARNED ? cap : __viaddmax_s16x2(cap, 0xFFFFFFFFu, 0u);
+        const uint32_t inner = Ck::template inner_of<LEARNED>(ck.smallest());
         auto steps = [&](auto ke) {
             constexpr int KE = decltype(ke)::value;
             for (int l = 0; l < nlev - 1; l++) {
@@ -944,7 +781,7 @@ __device__ __forceinline__ void layer_pair(const PairFrame& fr, const DevCode& c
                 ck.fold_shared(k, KE == 3 || ((sh >> k) & 1u));
         };
         constexpr int KS = Ck::K1 > 3 ? 3 : Ck::K1, KM = Ck::K1 > 5 ? 5 : Ck::K1,
-                      KL = Ck::K1 > 7 ? 7 : Ck::K1;
+                      KL = Ck::K1 > 7 ? 7 : Ck::K1, KN = Ck::K1 > 9 ? 9 : Ck::K1;
         const uint32_t lm = __reduce_or_sync(0xFFFFFFFFu, ck.inm | ck.outm);
         if (KS == Ck::K1 || (lm >> (KS + 1)) == 0)
             steps(std::integral_constant<int, KS>());
@@ -952,6 +789,8 @@ __device__ __forceinline__ void layer_pair(const PairFrame& fr, const DevCode& c
             steps(std::integral_constant<int, KM>());
         else if (KL == Ck::K1 || (lm >> (KL + 1)) == 0)
             steps(std::integral_constant<int, KL>());
+        else if (KN == Ck::K1 || (lm >> (KN + 1)) == 0)
+            steps(std::integral_constant<int, KN>());
         else
             steps(std::integral_constant<int, Ck::K1>());
     }
@@ -1015,13 +854,13 @@ __device__ void iterate_pair(const DevCode& c, const PairFrame& fr, void* msgv, 
         const int cnt = fr.eoff[i + 1] - fr.eoff[i];
         const int nlev = c.nlev[i];
         if (GDM > 0)
-            layer_pair<(GDM > 0 ? GDM : 2), false, LS, WIDE, LEARNED, PO, pair_key_form(A, B, GDM, LS)>(fr, c, i, cnt, nlev, rec, meta, fresh, msg,
+            layer_pair<(GDM > 0 ? GDM : 2), false, LS, WIDE, LEARNED, PO>(fr, c, i, cnt, nlev, rec, meta, fresh, msg,
                                                                            lA, lB, r0, r1, o0, o1);
         else if (A == B || cnt == A)
-            layer_pair<A + 2, true, LS, WIDE, LEARNED, PO, pair_key_form(A, B, GDM, LS)>(fr, c, i, cnt, nlev, rec, meta, fresh, msg, lA, lB, r0, r1,
+            layer_pair<A + 2, true, LS, WIDE, LEARNED, PO>(fr, c, i, cnt, nlev, rec, meta, fresh, msg, lA, lB, r0, r1,
                                                            o0, o1);
         else
-            layer_pair<B + 2, true, LS, WIDE, LEARNED, PO, pair_key_form(A, B, GDM, LS)>(fr, c, i, cnt, nlev, rec, meta, fresh, msg, lA, lB, r0, r1,
+            layer_pair<B + 2, true, LS, WIDE, LEARNED, PO>(fr, c, i, cnt, nlev, rec, meta, fresh, msg, lA, lB, r0, r1,
                                                            o0, o1);
         /* (i - 1, j) is final for this iteration; (i, j) goes to the next
          * layer, or, for the last layer, to the check (0, j + 1) */
@@ -1043,12 +882,12 @@ __device__ void iterate_pair(const DevCode& c, const PairFrame& fr, void* msgv, 
 static __device__ void store_lane(const DevCode& c, const PairFrame& fr, int h, uint8_t* __restrict__ dst)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int8_t* b = (const int8_t*)fr.post + h;
+    const uint8_t* b = (const uint8_t*)fr.post + h;
     const int nchunks = (c.kldpc + 31) / 32;
     for (int ch = warp; ch < nchunks; ch += nw) {
         const int v = ch * 32 + lane;
-        const int x = v < c.kldpc ? b[2 * v] : 0;
-        const unsigned m = __ballot_sync(0xFFFFFFFFu, x < 0);
+        const int x = v < c.kldpc ? b[2 * v] : 0x80;
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, x < 0x80);
         const unsigned rr = __byte_perm(__brev(m), 0, 0x0123);
         if (lane < 4 && 4 * ch + lane < c.nbytes)
             dst[4 * ch + lane] = (uint8_t)(rr >> (8 * lane));
@@ -1144,7 +983,7 @@ __device__ __forceinline__ void stream_frames(const DecodeParams& p, const DevCo
         }
         if (s_frame[0] < 0 && s_frame[1] < 0)
             break;
-        const int fail = syndrome_pair<PO, pair_key_form(A, B, GDM, LS)>(c, fr, &s_flag, s_row);
+        const int fail = syndrome_pair<PO>(c, fr, &s_flag, s_row);
         /* lanes whose frame is done: results out, refill */
         int done = 0;
         for (int h = 0; h < 2; h++) {
@@ -1201,7 +1040,7 @@ __global__ void __launch_bounds__(384, PM ? 2 : 1) k_decode_pair(DecodeParams p)
     void* msg = (char*)p.msg + (size_t)blockIdx.x * p.msg_stride;
     /* the parity words follow the message records in this CTA's slab */
     uint16_t* gpar = (uint16_t*)((char*)msg + (((size_t)c.R * (WIDE ? 16 : 8) + 15) & ~(size_t)15));
-    const PairFrame fr = stage_pair<PO, pair_key_form(A, B, GDM, LS)>(c, smem, gpar);
+    const PairFrame fr = stage_pair<PO>(c, smem, gpar);
     const int lT = stage_learn(p.learn, p.learn_class, p.learn_iters);
     const int nframes = p.nframes_dev ? *p.nframes_dev : p.nframes;
     const int t = threadIdx.x;
@@ -1235,7 +1074,7 @@ __global__ void __launch_bounds__(384, PM ? 2 : 1) k_decode_pair(DecodeParams p)
             int it = 0;
             bool ok = true;
             for (;;) {
-                const int fail = syndrome_pair<PO, pair_key_form(A, B, GDM, LS)>(c, fr, &s_flag, s_row);
+                const int fail = syndrome_pair<PO>(c, fr, &s_flag, s_row);
                 if (t == 0)
                     s_flag = 0; /* read again only after later barriers */
                 const int v = pair_team_vote(sync + 2 * it, M, fail != 0, p.err,
