@@ -58,17 +58,19 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel)
 }
 /* 0xFFFF in each lane whose bit 15 is set */
 __device__ __forceinline__ uint32_t lmask(uint32_t v) { return prmt(v, 0, 0xBB99); }
-/* 16-bit shared-memory accesses at a 32-bit shared address */
+/* 16-bit shared-memory accesses at a 32-bit shared address, to and from whole
+ * registers (a 16-bit register would cost a conversion on either side) */
 __device__ __forceinline__ uint32_t lds16(uint32_t a)
 {
-    unsigned short v;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
+    uint32_t v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(a));
     return v;
 }
 __device__ __forceinline__ void sts16(uint32_t a, uint32_t v)
 {
-    asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((unsigned short)v));
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "r"(v));
 }
+
 /*
  * One check node (i, j) for both lanes, on one thread: link slots
  * k = 0 .. S-1.  Slot 0 is the parity bit, slot 1 the previous parity bit
@@ -112,9 +114,9 @@ __device__ __forceinline__ uint32_t learned_lut(uint32_t c, uint32_t t)
 
 /*
  * Values are halves in units of 1/256, exact: a posterior P is kept as the byte
- * u = P + 128, which one PRMT makes the half 1024 + u, and
- *     x = sat((1024 + u)/256 - (4 + m)) - 1/2 = (P - m)/256,
- * the saturating fused multiply-add being the clamp at -128 and one minimum
+ * u = P + 128, which one PRMT makes the half 4 + u/256, and
+ *     x = sat((4 + u/256) - (4 + m)) - 1/2 = (P - m)/256,
+ * the saturating add being the clamp at -128 and one minimum
  * the clamp at 127 (255/256 before the half is taken off).  |x| is an operand
  * modifier of the minimum, a link's message magnitude is a fused multiply-add
  * of the comparison's 1.0, min0 + f (min1 - min0), its sign one LOP3.  The
@@ -135,40 +137,33 @@ __device__ __forceinline__ uint32_t learned_lut(uint32_t c, uint32_t t)
  */
 __device__ __forceinline__ __half2 h2(uint32_t a) { return *(const __half2*)&a; }
 __device__ __forceinline__ uint32_t u2(__half2 a) { return *(const uint32_t*)&a; }
-constexpr uint32_t kHUnit = 0x1C001C00u;   /* 1/256 */
 constexpr uint32_t kH127 = 0x37F037F0u;    /* 127/256 */
-constexpr uint32_t kH255 = 0x3BF83BF8u;    /* 255/256 */
 constexpr uint32_t kHHalf = 0x38003800u;   /* 1/2 */
 constexpr uint32_t kH31 = 0x2FC02FC0u;     /* 31/256 */
 constexpr uint32_t kH32 = 0x30003000u;     /* 32/256 */
-constexpr uint32_t kHFour = 0x44004400u;   /* 4 */
-constexpr uint32_t kH256 = 0x5C005C00u;    /* 256 */
-constexpr uint32_t kH1024 = 0x64006400u;   /* 1024: its low bits hold an integer below 1024 */
+constexpr uint32_t kHFour = 0x44004400u;   /* 4: its low byte counts in 1/256 */
+constexpr uint32_t kH255 = 0x3BF83BF8u;    /* 255/256 */
+constexpr uint32_t kHNegFour = 0xC400C400u;
 constexpr uint32_t kHOne = 0x3C003C00u;    /* above every magnitude */
 constexpr uint32_t kHSign = 0x80008000u;
 constexpr uint32_t kHNegUnit = 0x9C009C00u; /* -1/256 */
 
-/* integers below 1024 in both lanes as halves in 1/256, and back */
-__device__ __forceinline__ uint32_t h_of_int(uint32_t v)
+__device__ __forceinline__ uint32_t h_add(uint32_t a, uint32_t b) { return u2(__hadd2(h2(a), h2(b))); }
+/* bytes in both lanes as halves in 1/256, and back */
+__device__ __forceinline__ uint32_t h_of_int(uint32_t v) { return h_add(v | kHFour, kHNegFour); }
+__device__ __forceinline__ uint32_t h_to_int(uint32_t v) { return h_add(v, kHFour) & 0x00FF00FFu; }
+/* x from a posterior word (two bytes u), whose halves' upper bytes come from
+ * four (0x44 in its byte 1), and minus 4 minus the message */
+__device__ __forceinline__ uint32_t h_input(uint32_t raw, uint32_t four, uint32_t cm)
 {
-    return u2(__hfma2(h2(v | kH1024), h2(kHUnit), h2(kHFour | kHSign)));
-}
-__device__ __forceinline__ uint32_t h_to_int(uint32_t v)
-{
-    return u2(__hfma2(h2(v), h2(kH256), h2(kH1024))) & 0x03FF03FFu;
-}
-/* x from a posterior word (two bytes u) and minus 4 minus the message */
-__device__ __forceinline__ uint32_t h_input(uint32_t raw, uint32_t cm)
-{
-    const uint32_t z = u2(__hfma2_sat(h2(prmt(raw, 0x64646464u, 0x4140)), h2(kHUnit), h2(cm)));
-    return u2(__hsub2(__hmin2(h2(z), h2(kH255)), h2(kHHalf)));
+    const __half2 z = __hadd2_sat(h2(prmt(raw, four, 0x5150)), h2(cm));
+    return u2(__hsub2(__hmin2(z, h2(kH255)), h2(kHHalf)));
 }
 /* the new posterior's two bytes from x and the message */
 __device__ __forceinline__ uint32_t h_output(uint32_t x, uint32_t m)
 {
-    const __half2 z = __hadd2_sat(h2(x), __hadd2(h2(m), h2(kHHalf)));
-    const uint32_t q = u2(__hfma2(__hmin2(z, h2(kH255)), h2(kH256), h2(kH1024)));
-    return prmt(q, 0, 0x0020);
+    const __half2 z = __hmin2(__hadd2_sat(h2(x), h2(h_add(m, kHHalf))), h2(kH255));
+    return prmt(h_add(u2(z), kHFour), 0, 0x0020);
 }
 __device__ __forceinline__ uint32_t h_abs(uint32_t x) { return u2(__habs2(h2(x))); }
 __device__ __forceinline__ uint32_t h_min(uint32_t a, uint32_t b) { return u2(__hmin2(h2(a), h2(b))); }
@@ -228,10 +223,10 @@ struct PairCheck {
         sgn = rec.y & ~fresh;
         if constexpr (WIDE) {
             sgn1 = rec.z & ~fresh;
-            idxh = (rec.w & ~fresh) | kH1024;
+            idxh = (rec.w & ~fresh) | kHFour;
         } else {
             sgn1 = 0;
-            idxh = ((w0 >> 12) & 0x000F000Fu) | kH1024;
+            idxh = ((w0 >> 12) & 0x000F000Fu) | kHFour;
         }
         om0 = h_of_int(w0 & 0x003F003Fu);
         omd = u2(__hsub2(h2(h_of_int((w0 >> 6) & 0x003F003Fu)), h2(om0)));
@@ -242,10 +237,10 @@ struct PairCheck {
     /* minus 4 minus the old message of slot k: its magnitude with its sign, at most 31 */
     __device__ __forceinline__ uint32_t unmsg(int k) const
     {
-        const uint32_t mag = u2(__hfma2(h_eq(idxh, kH1024 + (uint32_t)k * 0x00010001u), h2(omd), h2(om0)));
+        const uint32_t mag = u2(__hfma2(h_eq(idxh, kHFour + (uint32_t)k * 0x00010001u), h2(omd), h2(om0)));
         const int s = (k & 15) >> 1;
         const uint32_t m = ((((k < 16 ? sgn : sgn1) << ((k & 1) ? s : s + 8)) & kHSign) ^ mag);
-        return u2(__hsub2(h2(kHFour | kHSign), __hmin2(h2(m), h2(kH31))));
+        return u2(__hsub2(h2(kHNegFour), __hmin2(h2(m), h2(kH31))));
     }
 
     __device__ __forceinline__ void fold(uint32_t a)
@@ -261,7 +256,7 @@ struct PairCheck {
         auto slot = [&](int k) {
             const uint32_t m = unmsg(k);
             const uint32_t raw = PO && k < 2 ? (k == 0 ? r0 : r1) : lds16(addr[k]);
-            uint32_t v = h_input(raw, m);
+            uint32_t v = h_input(raw, idxh, m);
             const bool maybe_shared = LEV && k >= K0 && k <= K1;
             if (!EXACT || k == 1) { /* a slot that can be absent: above every minimum, positive */
                 v = ((live >> k) & 1u) ? v : kHOne;
@@ -299,7 +294,7 @@ struct PairCheck {
         }
         live = inm = outm = 0;
         om0 = omd = sgn = sgn1 = 0;
-        idxh = kH1024;
+        idxh = kHFour;
         min0 = min1 = kHOne;
         sg = mn0 = mnd = recw = 0;
     }
@@ -325,14 +320,14 @@ struct PairCheck {
         __half2 idxs[CH];
 #pragma unroll
         for (int q = 0; q < CH; q++)
-            idxs[q] = h2(kH1024);
+            idxs[q] = h2(kHFour);
 #pragma unroll
         for (int k = 0; k < S; k++) {
             const __half2 f = h_eq(h_abs(x[k]), min0);
             const uint32_t m = u2(__hfma2(f, h2(mnd), h2(mn0))) ^ (x[k] & kHSign);
             const uint32_t nv = h_output(x[k], m);
             __half2& idx = idxs[k % CH];
-            idx = __hfma2(f, __hsub2(h2(kH1024 + (uint32_t)k * 0x00010001u), idx), idx);
+            idx = __hfma2(f, __hsub2(h2(kHFour + (uint32_t)k * 0x00010001u), idx), idx);
             if (PO && k < 2)
                 (k == 0 ? o0 : o1) = nv;
             else if (EXACT && k > K1 && k != 1)
@@ -363,7 +358,7 @@ struct PairCheck {
 
     /* shared links, see level_step */
     static __device__ __forceinline__ uint32_t none() { return kHOne; }
-    static __device__ __forceinline__ uint32_t value(uint32_t raw, uint32_t m) { return h_input(raw, m); }
+    __device__ __forceinline__ uint32_t value(uint32_t raw, uint32_t m) const { return h_input(raw, idxh, m); }
     template <bool LEARNED>
     static __device__ __forceinline__ uint32_t inner_of(uint32_t smallest)
     {
@@ -602,7 +597,7 @@ __device__ __forceinline__ void read_late(Ck& ck, bool mine)
     const uint32_t im = mine ? ck.inm : 0u;
 #pragma unroll
     for (int k = Ck::K0; k <= KE; k++) {
-        const uint32_t v = Ck::value(lds16(ck.addr[k]), ck.x[k]);
+        const uint32_t v = ck.value(lds16(ck.addr[k]), ck.x[k]);
         ck.x[k] = (im >> k) & 1u ? v : ck.x[k];
     }
 }
@@ -614,7 +609,7 @@ __device__ __forceinline__ void level_step(Ck& ck, uint32_t inner, bool mine, bo
     const uint32_t im = mine ? ck.inm : 0u, om = mine ? ck.outm : 0u, sh = ck.inm | ck.outm;
     auto read = [&](int k) {
         if (late) {
-            const uint32_t v = Ck::value(lds16(ck.addr[k]), ck.x[k]);
+            const uint32_t v = ck.value(lds16(ck.addr[k]), ck.x[k]);
             ck.x[k] = (im >> k) & 1u ? v : ck.x[k];
         }
         return Ck::template mag<LEARNED>(ck.x[k]);
