@@ -35,7 +35,11 @@ using namespace drxg;
 
 namespace {
 
-constexpr int kSideStreams = 4;
+/* Branches of the per-code graph.  A code's launch lasts as long as its slowest
+ * frames, which leave most of its CTAs idle; with four branches a 2048-frame
+ * batch of 21 codes (49 CTAs each) took 9.93 ms, with eight 9.49, with sixteen
+ * 8.73 and with 24 8.83; at 16384 frames 56.2, 54.6, 54.4 and 55.3 ms. */
+constexpr int kSideStreams = 16;
 
 }  // namespace
 
