@@ -25,22 +25,23 @@
 
 namespace drxg {
 
-/* the shapes behind the switch: (A, B, GDM, LS) of the one-CTA frame-pair
+/* the shapes behind the switch: (A, B, EVERY, LS) of the one-CTA frame-pair
  * kernels that pair_kernel_id picks for the DVB-S2 codes */
 #define DRXG_MIX_SHAPES(X)                                                                               \
     X(0, 1, 2, 0, 1) X(1, 2, 2, 0, 1) X(2, 3, 3, 0, 1) X(3, 4, 4, 0, 1) X(4, 5, 5, 0, 1) X(5, 8, 8, 0, 2) \
     X(6, 9, 9, 0, 2) X(7, 12, 12, 0, 2) X(8, 9, 9, 0, 3) X(9, 16, 16, 0, 4) X(10, 20, 20, 0, 3)          \
-    X(11, 25, 25, 0, 6) X(12, 28, 28, 0, 4) X(13, 1, 1, 7, 1) X(14, 1, 1, 14, 3) X(15, 1, 1, 22, 5) X(16, 25, 25, 0, 3)
+    X(11, 25, 25, 0, 6) X(12, 28, 28, 0, 4) X(13, 2, 5, 1, 1) X(14, 7, 11, 1, 2) X(15, 14, 17, 1, 5)     \
+    X(16, 25, 25, 0, 3) X(17, 9, 11, 1, 3)
 
 /* One code's frames with its shape: its tables staged,
  * then the streaming loop of the frame-pair kernel. */
-template <int A, int B, int GDM, int LS>
+template <int A, int B, int EVERY, int LS>
 __device__ __noinline__ void mix_code_frames(const DecodeParams& p, const DevCode& c, char* smem, void* msg,
                                              PairLanes& st)
 {
     const PairFrame fr = stage_pair<false>(c, smem, nullptr);
     __syncthreads();
-    stream_frames<A, B, GDM, LS, false>(p, c, fr, msg, 0, p.nframes, st);
+    stream_frames<A, B, EVERY, LS, false>(p, c, fr, msg, 0, p.nframes, st);
 }
 
 /* The code with the most work left (frames not yet taken x edges), -1 if none. */
@@ -109,13 +110,13 @@ __global__ void __launch_bounds__(384, 1) k_decode_mix_pair(MixPairParams mp)
     }
 }
 
-/* The shape index of a one-CTA frame-pair kernel (a, b, gdm, ls), -1 if the
+/* The shape index of a one-CTA frame-pair kernel (a, b, every, ls), -1 if the
  * switch does not hold it. */
-int mix_pair_shape(int a, int b, int gdm, int ls)
+int mix_pair_shape(int a, int b, int every, int ls)
 {
     int k = -1;
 #define DRXG_MIX_FIND(i, aa, bb, gg, ll)                          \
-    if (gg == gdm && ll == ls && (gg > 0 || (aa == a && bb == b))) \
+    if (gg == every && ll == ls && aa == a && bb == b) \
         k = k < 0 ? i : k;
     DRXG_MIX_SHAPES(DRXG_MIX_FIND)
 #undef DRXG_MIX_FIND

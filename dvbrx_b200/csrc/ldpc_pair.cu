@@ -39,9 +39,11 @@ const PairKernel* pair_kernel_part(int part, int* n)
 
 /* Every instantiated kernel, the parts in order (the index is the kernel
  * id).  Pair kernels by information-link counts (A, B): every pair of the
- * DVB-S2, S2X and T2 codes, plus predicated kernels for the codes whose
- * layers have more than two different counts (degree bounds 7, 11, 14, 22,
- * 32); LS: half the shared slots the kernel carries (none for the shapes of
+ * DVB-S2, S2X and T2 codes, and for the short codes with more than two counts
+ * (1/2, 3/4, 4/5, 5/6) kernels with a node for every count from A to B (a node
+ * of the largest degree with predicated slots before: short 1/2 0.071 -> 0.059
+ * us per frame-iteration, 3/4 0.060 -> 0.050, 4/5 0.057 -> 0.053, 5/6 0.139 ->
+ * 0.126); LS: half the shared slots the kernel carries (none for the shapes of
  * the S2X codes alone, which then hold no level code: 18/30 0.339 -> 0.305 us
  * per frame-iteration; one or two for most levelled codes, three to six from
  * normal 4/5, short 3/5 and 4/5 up); residency
@@ -78,19 +80,19 @@ size_t decode_pair_msg_bytes(int R, int kid)
     if (kid < 0 || kid >= (int)kernels().size())
         return 0;
     const PairKernel& k = kernels()[kid];
-    const int dm = k.gdm > 0 ? k.gdm : k.b + 2;
+    const int dm = k.b + 2;
     const size_t rec = a16h((size_t)R * (dm > 16 ? sizeof(uint4) : sizeof(uint2)));
     return rec + (k.pm == 2 ? a16h(sizeof(uint16_t) * (size_t)(R - kQCp)) : 0);
 }
 
-bool pair_kernel_shape(int kid, int* a, int* b, int* gdm, int* ls, int* pm)
+bool pair_kernel_shape(int kid, int* a, int* b, int* every, int* ls, int* pm)
 {
     if (kid < 0 || kid >= (int)kernels().size())
         return false;
     const PairKernel& k = kernels()[kid];
     *a = k.a;
     *b = k.b;
-    *gdm = k.gdm;
+    *every = k.every;
     *ls = k.ls;
     *pm = k.pm;
     return true;
@@ -104,7 +106,7 @@ int pair_kernel_twin(int kid, int pm)
     const PairKernel& k = kernels()[kid];
     for (int t = 0; t < (int)kernels().size(); t++) {
         const PairKernel& u = kernels()[t];
-        if (u.pm == pm && u.a == k.a && u.b == k.b && u.gdm == k.gdm && u.ls == k.ls)
+        if (u.pm == pm && u.a == k.a && u.b == k.b && u.every == k.every && u.ls == k.ls)
             return t;
     }
     return -1;
@@ -133,13 +135,9 @@ int pair_kernel_id(const Code& c)
         const int n = c.eoff[i + 1] - c.eoff[i];
         other |= n != lo && n != hi;
     }
-    if (!other)
-        for (int k = 0; k < (int)kernels().size(); k++)
-            if (kernels()[k].pm == 0 && kernels()[k].gdm == 0 && kernels()[k].a == lo &&
-                kernels()[k].b == hi && kernels()[k].ls >= ls)
-                return k;
     for (int k = 0; k < (int)kernels().size(); k++)
-        if (kernels()[k].pm == 0 && kernels()[k].gdm >= c.deg_max && kernels()[k].ls >= ls)
+        if (kernels()[k].pm == 0 && kernels()[k].every == other && kernels()[k].a == lo && kernels()[k].b == hi &&
+            kernels()[k].ls >= ls)
             return k;
     return -1;
 }

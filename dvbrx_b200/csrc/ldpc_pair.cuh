@@ -75,8 +75,7 @@ __device__ __forceinline__ void sts16(uint32_t a, uint32_t v)
  * One check node (i, j) for both lanes, on one thread: link slots
  * k = 0 .. S-1.  Slot 0 is the parity bit, slot 1 the previous parity bit
  * (absent for (0, 0)), 2 + e information entry e of the layer.  DM is the
- * node degree (EXACT) or a bound on it (the degree is then a run-time
- * value).  The node state lives in registers across the phases of its layer
+ * node degree.  The node state lives in registers across the phases of its layer
  * (see layer_pair).  Slot masks and the message index keep slot k at bit k.
  *
  * The full passes run every slot without branches: a slot that is not a link,
@@ -178,7 +177,7 @@ __device__ __forceinline__ uint32_t h_offset(uint32_t a)
 /* learned magnitudes of capped minimums c */
 __device__ __forceinline__ uint32_t h_learned(uint32_t c, uint32_t lp) { return h_of_int(learned_lut(h_to_int(c), lp)); }
 
-template <int DM, bool EXACT, int LS, bool WIDE, bool PO>
+template <int DM, int LS, bool WIDE, bool PO>
 struct PairCheck {
     static_assert(DM <= (WIDE ? 32 : 16), "degree above the record's slots");
     using Rec = PairRec<WIDE>;
@@ -192,13 +191,12 @@ struct PairCheck {
     uint32_t min0, min1, sg;            /* smallest magnitudes, sign parity (bit 15 / 31) */
     uint32_t mn0, mnd, recw;            /* outgoing magnitudes with the parity's sign (set by finish), record word */
 
-    __device__ __forceinline__ void setup(const int2* __restrict__ ent, int cnt, int K, int q, int i, int j,
+    __device__ __forceinline__ void setup(const int2* __restrict__ ent, int K, int q, int i, int j,
                                           Rec rec, uint32_t fresh, unsigned long long meta, uint32_t sbase)
     {
-        const int D = EXACT ? DM : cnt + 2;
         const int pc = K + kQCp * i + j;
         const int pp = i ? pc - kQCp : K + kQCp * (q - 1) + j - 1;
-        uint32_t lv = (1u << D) - 1u;
+        uint32_t lv = (uint32_t)((1ull << DM) - 1ull);
         if ((i | j) == 0)
             lv &= ~2u;
         live = lv;
@@ -210,10 +208,9 @@ struct PairCheck {
             if (k < 2) {
                 addr[k] = PO ? 0u : sbase + 2u * (uint32_t)(k == 0 ? pc : pp);
             } else {
-                /* a slot past the degree takes the last link's address: read, never used.
-                 * Link of check j: word (j - a) mod 360 of the group, as min(u, u + 720)
+                /* link of check j: word (j - a) mod 360 of the group, as min(u, u + 720)
                  * over unsigned byte offsets u = 2 j - 2 a */
-                const int2 e = ent[(EXACT ? k : min(k, D - 1)) - 2];
+                const int2 e = ent[k - 2];
                 const uint32_t u = tj + (uint32_t)e.y;
                 addr[k] = (uint32_t)e.x + __viaddmin_u32(u, 2u * kQCp, u);
             }
@@ -258,7 +255,7 @@ struct PairCheck {
             const uint32_t raw = PO && k < 2 ? (k == 0 ? r0 : r1) : lds16(addr[k]);
             uint32_t v = h_input(raw, idxh, m);
             const bool maybe_shared = LEV && k >= K0 && k <= K1;
-            if (!EXACT || k == 1) { /* a slot that can be absent: above every minimum, positive */
+            if (k == 1) { /* a slot that can be absent: above every minimum, positive */
                 v = ((live >> k) & 1u) ? v : kHOne;
             }
             x[k] = maybe_shared && ((inm >> k) & 1u) ? m : v; /* a late slot waits for its level */
@@ -330,7 +327,7 @@ struct PairCheck {
             idx = __hfma2(f, __hsub2(h2(kHFour + (uint32_t)k * 0x00010001u), idx), idx);
             if (PO && k < 2)
                 (k == 0 ? o0 : o1) = nv;
-            else if (EXACT && k > K1 && k != 1)
+            else if (k > K1 && k != 1)
                 sts16(addr[k], nv); /* every slot past K1 is a link written here */
             else if ((wm >> k) & 1u)
                 sts16(addr[k], nv);
@@ -724,8 +721,8 @@ __device__ __forceinline__ void level_step(Ck& ck, uint32_t inner, bool mine, bo
  * layer share, so the wavefront levels carry just those links.  Unlevelled
  * layers take one pass.
  */
-template <int DM, bool EXACT, int LS, bool WIDE, bool LEARNED, bool PO>
-__device__ __forceinline__ void layer_pair(const PairFrame& fr, const DevCode& c, int i, int cnt, int nlev,
+template <int DM, int LS, bool WIDE, bool LEARNED, bool PO>
+__device__ __forceinline__ void layer_pair(const PairFrame& fr, const DevCode& c, const int2* ent, int i, int nlev,
                                            PairRec<WIDE> rec, unsigned long long meta, uint32_t fresh,
                                            PairRec<WIDE>* __restrict__ msg, int lA, int lB, uint32_t r0,
                                            uint32_t r1, uint32_t& o0, uint32_t& o1)
@@ -735,12 +732,12 @@ __device__ __forceinline__ void layer_pair(const PairFrame& fr, const DevCode& c
     const int j = t;
     /* the check's learned class table (an index into s_learn_lut) */
     auto lclass = [&]() {
-        return LEARNED ? 128u * (uint32_t)s_learn_cls[(EXACT ? DM : cnt + 2) - ((i | j) == 0)] : 0u;
+        return LEARNED ? 128u * (uint32_t)s_learn_cls[DM - ((i | j) == 0)] : 0u;
     };
-    using Ck = PairCheck<DM, EXACT, LS, WIDE, PO>;
+    using Ck = PairCheck<DM, LS, WIDE, PO>;
     Ck ck;
     if (active) {
-        ck.setup(fr.ent + fr.eoff[i], cnt, c.K, c.q, i, j, rec, fresh, meta,
+        ck.setup(ent, c.K, c.q, i, j, rec, fresh, meta,
                  (uint32_t)__cvta_generic_to_shared(fr.post));
         if (LS > 0 && nlev > 1)
             ck.template read_all<true>(fr.post, r0, r1);
@@ -796,19 +793,38 @@ __device__ __forceinline__ void layer_pair(const PairFrame& fr, const DevCode& c
     __syncthreads();
 }
 
+/* Layer i with the exact-degree node of its count, one of A, A + STEP .. B */
+template <int A, int B, int STEP, int LS, bool WIDE, bool LEARNED, bool PO>
+__device__ __forceinline__ void layer_of_count(const PairFrame& fr, const DevCode& c, const int2* ent, int i, int cnt, int nlev,
+                                               PairRec<WIDE> rec, unsigned long long meta, uint32_t fresh,
+                                               PairRec<WIDE>* __restrict__ msg, int lA, int lB, uint32_t r0,
+                                               uint32_t r1, uint32_t& o0, uint32_t& o1)
+{
+    if (A == B || cnt == A)
+        layer_pair<A + 2, LS, WIDE, LEARNED, PO>(fr, c, ent, i, nlev, rec, meta, fresh, msg, lA, lB, r0, r1, o0,
+                                                       o1);
+    else if constexpr (A < B)
+        layer_of_count<A + STEP, B, STEP, LS, WIDE, LEARNED, PO>(fr, c, ent, i, cnt, nlev, rec, meta, fresh, msg, lA, lB,
+                                                                 r0, r1, o0, o1);
+}
+
 /* One decoding iteration: the layers in order; each layer's messages and
  * level metadata are fetched one layer ahead.  The kernel is compiled for
  * the two information-link counts A <= B of its codes (exact-degree check
- * nodes), or, with GDM > 0, for any count up to GDM - 2 (predicated). */
-template <int A, int B, int GDM, int LS, bool LEARNED, bool PO>
+ * nodes), or, with EVERY, for every count from A to B. */
+template <int A, int B, int EVERY, int LS, bool LEARNED, bool PO>
 __device__ void iterate_pair(const DevCode& c, const PairFrame& fr, void* msgv, uint32_t fresh, int lA, int lB)
 {
-    constexpr bool WIDE = (GDM > 0 ? GDM : B + 2) > 16;
+    constexpr bool WIDE = B + 2 > 16;
     using Rec = PairRec<WIDE>;
     Rec* __restrict__ msg = (Rec*)msgv;
     const int t = threadIdx.x;
     const int j = t;
     const bool active = t < kQCp;
+    /* the next layer's levels, read a layer ahead: read in their own layer, every warp
+     * waited for them at its start (normal 2/3 0.279 -> 0.242 us per frame-iteration,
+     * 1/2 0.264 -> 0.223, together with entries at A i where A = B) */
+    int nl = c.nlev[0];
     Rec rn{};
     unsigned long long mn = 0;
     /* PO: the words of parity bits (i, j) and (i + 1, j) for layers i and
@@ -846,17 +862,13 @@ __device__ void iterate_pair(const DevCode& c, const PairFrame& fr, void* msgv, 
                 pnext2 = fr.gpar[kQCp * (i + 2) + j];
             r1 = i ? carry : (j ? fr.wrap[j - 1] : 0u);
         }
-        const int cnt = fr.eoff[i + 1] - fr.eoff[i];
-        const int nlev = c.nlev[i];
-        if (GDM > 0)
-            layer_pair<(GDM > 0 ? GDM : 2), false, LS, WIDE, LEARNED, PO>(fr, c, i, cnt, nlev, rec, meta, fresh, msg,
-                                                                           lA, lB, r0, r1, o0, o1);
-        else if (A == B || cnt == A)
-            layer_pair<A + 2, true, LS, WIDE, LEARNED, PO>(fr, c, i, cnt, nlev, rec, meta, fresh, msg, lA, lB, r0, r1,
-                                                           o0, o1);
-        else
-            layer_pair<B + 2, true, LS, WIDE, LEARNED, PO>(fr, c, i, cnt, nlev, rec, meta, fresh, msg, lA, lB, r0, r1,
-                                                           o0, o1);
+        const int first = A == B ? A * i : fr.eoff[i];
+        const int cnt = A == B ? A : fr.eoff[i + 1] - first;
+        const int2* ent = fr.ent + first;
+        const int nlev = nl;
+        nl = c.nlev[i + 1 < c.q ? i + 1 : i];
+        layer_of_count<A, B, EVERY ? 1 : B - A, LS, WIDE, LEARNED, PO>(fr, c, ent, i, cnt, nlev, rec, meta, fresh, msg,
+                                                                       lA, lB, r0, r1, o0, o1);
         /* (i - 1, j) is final for this iteration; (i, j) goes to the next
          * layer, or, for the last layer, to the check (0, j + 1) */
         if (PO && active) {
@@ -896,6 +908,8 @@ static __device__ void store_lane(const DevCode& c, const PairFrame& fr, int h, 
 static __device__ int pair_team_vote(unsigned* slot, int M, bool fail, int* err, int limit, bool skip)
 {
     __shared__ int s_res;
+    if (M == 1 && !skip) /* a team of one has nobody to ask */
+        return fail ? 0 : 1;
     if (threadIdx.x == 0) {
         unsigned* arrive = slot;
         unsigned* fails = slot + 1;
@@ -941,7 +955,7 @@ struct PairLanes {
  * work item k is row p.rows[k], or k), so a converged frame never waits for
  * its neighbour.  The CTA's tables are staged (fr) and its lane state
  * initialised (frames -1, both lanes to reload, flag 0, rows 0). */
-template <int A, int B, int GDM, int LS, bool PO>
+template <int A, int B, int EVERY, int LS, bool PO>
 __device__ __forceinline__ void stream_frames(const DecodeParams& p, const DevCode& c, const PairFrame& fr, void* msg,
                                               int lT, int nframes, PairLanes& st)
 {
@@ -1004,10 +1018,10 @@ __device__ __forceinline__ void stream_frames(const DecodeParams& p, const DevCo
         if (done)
             continue; /* reload, then check the new frames first */
         if (lT)
-            iterate_pair<A, B, GDM, LS, true, PO>(c, fr, msg, fresh, learn_row(s_iter[0], lT),
+            iterate_pair<A, B, EVERY, LS, true, PO>(c, fr, msg, fresh, learn_row(s_iter[0], lT),
                                                   learn_row(s_iter[1], lT));
         else
-            iterate_pair<A, B, GDM, LS, false, PO>(c, fr, msg, fresh, -1, -1);
+            iterate_pair<A, B, EVERY, LS, false, PO>(c, fr, msg, fresh, -1, -1);
         fresh = 0;
         if (t == 0) {
             s_iter[0]++;
@@ -1020,7 +1034,7 @@ __device__ __forceinline__ void stream_frames(const DecodeParams& p, const DevCo
 /* PM: 0 one resident CTA per SM; 1 two (80 registers), for codes whose
  * posteriors leave room for two (short frames); 2 two, with the parity
  * posteriors out of shared memory (PO: normal frames up to rate 4/5) */
-template <int A, int B, int GDM, int LS, int PM>
+template <int A, int B, int EVERY, int LS, int PM>
 __global__ void __launch_bounds__(384, PM ? 2 : 1) k_decode_pair(DecodeParams p)
 {
     constexpr bool PO = PM == 2;
@@ -1031,7 +1045,7 @@ __global__ void __launch_bounds__(384, PM ? 2 : 1) k_decode_pair(DecodeParams p)
     int& s_reload = ((PairLanes*)s_lanes)->reload;
     int* s_row = ((PairLanes*)s_lanes)->row;
     const DevCode c = *p.code;
-    constexpr bool WIDE = (GDM > 0 ? GDM : B + 2) > 16;
+    constexpr bool WIDE = B + 2 > 16;
     void* msg = (char*)p.msg + (size_t)blockIdx.x * p.msg_stride;
     /* the parity words follow the message records in this CTA's slab */
     uint16_t* gpar = (uint16_t*)((char*)msg + (((size_t)c.R * (WIDE ? 16 : 8) + 15) & ~(size_t)15));
@@ -1078,7 +1092,7 @@ __global__ void __launch_bounds__(384, PM ? 2 : 1) k_decode_pair(DecodeParams p)
                 ok = v == 1;
                 if (v < 0 || ok || it >= p.max_iter)
                     break;
-                iterate_pair<A, B, GDM, LS, false, PO>(c, fr, msg, gfresh, -1, -1);
+                iterate_pair<A, B, EVERY, LS, false, PO>(c, fr, msg, gfresh, -1, -1);
                 gfresh = 0;
                 it++;
             }
@@ -1098,15 +1112,14 @@ __global__ void __launch_bounds__(384, PM ? 2 : 1) k_decode_pair(DecodeParams p)
         return;
     }
     PairLanes& st = *(PairLanes*)s_lanes;
-    stream_frames<A, B, GDM, LS, PO>(p, c, fr, msg, lT, nframes, st);
+    stream_frames<A, B, EVERY, LS, PO>(p, c, fr, msg, lT, nframes, st);
 }
 
 /* Pair kernels by information-link counts (A, B): every pair of the DVB-S2,
- * S2X and T2 codes, plus predicated kernels for the codes whose layers have
- * more than two different counts (degree bounds 7, 11, 14, 22, 32).  LS:
+ * S2X and T2 codes, or every count from A to B (every = 1).  LS:
  * half the shared slots the kernel carries. */
 struct PairKernel {
-    int a, b, gdm, ls, pm, threads;
+    int a, b, every, ls, pm, threads;
     const void* fn;
 };
 
@@ -1117,6 +1130,6 @@ const PairKernel* pair_kernel_part(int part, int* n);
 constexpr int kPairKernelParts = 6;
 
 /* launch bounds of a residency mode: 1 CTA per SM (mode 0) or two */
-#define DRXG_PAIR_KERNEL(a, b, gdm, ls, pm) { a, b, gdm, ls, pm, 384, (const void*)k_decode_pair<a, b, gdm, ls, pm> }
+#define DRXG_PAIR_KERNEL(a, b, every, ls, pm) { a, b, every, ls, pm, 384, (const void*)k_decode_pair<a, b, every, ls, pm> }
 
 }  // namespace drxg

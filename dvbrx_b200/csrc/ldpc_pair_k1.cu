@@ -15,11 +15,10 @@ static const PairKernel kPart[] = {
     DRXG_PAIR_KERNEL(25, 25, 0, 6, 0),
     DRXG_PAIR_KERNEL(27, 28, 0, 0, 0),
     DRXG_PAIR_KERNEL(28, 28, 0, 4, 0),
-    DRXG_PAIR_KERNEL(1, 1, 7, 1, 0),
-    DRXG_PAIR_KERNEL(1, 1, 11, 3, 0),
-    DRXG_PAIR_KERNEL(1, 1, 14, 3, 0),
-    DRXG_PAIR_KERNEL(1, 1, 22, 5, 0),
-    DRXG_PAIR_KERNEL(1, 1, 32, 6, 0),
+    DRXG_PAIR_KERNEL(2, 5, 1, 1, 0),
+    DRXG_PAIR_KERNEL(7, 11, 1, 2, 0),
+    DRXG_PAIR_KERNEL(9, 11, 1, 3, 0),
+    DRXG_PAIR_KERNEL(14, 17, 1, 5, 0),
 };
 
 const PairKernel* pair_kernel_part1(int* n)

@@ -10,14 +10,11 @@ static const PairKernel kPart[] = {
     DRXG_PAIR_KERNEL(12, 12, 0, 2, 2),
     DRXG_PAIR_KERNEL(9, 9, 0, 3, 1),
     DRXG_PAIR_KERNEL(9, 9, 0, 3, 2),
-    DRXG_PAIR_KERNEL(1, 1, 7, 1, 1),
-    DRXG_PAIR_KERNEL(1, 1, 7, 1, 2),
-    DRXG_PAIR_KERNEL(1, 1, 11, 3, 1),
-    DRXG_PAIR_KERNEL(1, 1, 11, 3, 2),
-    DRXG_PAIR_KERNEL(1, 1, 14, 3, 1),
-    DRXG_PAIR_KERNEL(1, 1, 14, 3, 2),
+    DRXG_PAIR_KERNEL(2, 5, 1, 1, 1),
+    DRXG_PAIR_KERNEL(7, 11, 1, 2, 1),
+    DRXG_PAIR_KERNEL(9, 11, 1, 3, 1),
+    DRXG_PAIR_KERNEL(14, 17, 1, 5, 1),
     DRXG_PAIR_KERNEL(16, 16, 0, 4, 2),
-    DRXG_PAIR_KERNEL(1, 1, 22, 5, 1),
     DRXG_PAIR_KERNEL(25, 25, 0, 6, 1),
 };
 

@@ -28,11 +28,11 @@ struct MixPairParams {
 };
 
 /* shape index of a one-CTA frame-pair kernel, -1 if the mixed kernel lacks it */
-int mix_pair_shape(int a, int b, int gdm, int ls);
+int mix_pair_shape(int a, int b, int every, int ls);
 int decode_mix_pair_ctas_per_sm(size_t smem);
 cudaError_t launch_decode_mix_pair(const MixPairParams& p, size_t smem, int grid, cudaStream_t stream);
 
-/* (a, b, gdm, ls, pm) of frame-pair kernel kid (ldpc_pair.cu); false if none */
-bool pair_kernel_shape(int kid, int* a, int* b, int* gdm, int* ls, int* pm);
+/* (a, b, every, ls, pm) of frame-pair kernel kid (ldpc_pair.cu); false if none */
+bool pair_kernel_shape(int kid, int* a, int* b, int* every, int* ls, int* pm);
 
 }  // namespace drxg
