@@ -279,7 +279,9 @@ __global__ void __launch_bounds__(32 * kRemMaxWarps) k_bch_remainder(BchBatch b,
 #pragma unroll
                 for (int w = 0; w < NW; w++)
                     b.rem[(size_t)f * NW + w] = r[w];
-                b.queue[atomicAdd(b.count, 1)] = f;
+                const int at = atomicAdd(b.count, 1);
+                if (at < b.nframes) /* always, unless an earlier batch's correction never ran */
+                    b.queue[at] = f;
             }
         }
     }
@@ -431,7 +433,7 @@ __global__ void __launch_bounds__(kFixThreads, 4) k_bch_correct(BchBatch b)
     __shared__ FixShared s;
     const BchDev& c = b.c;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int n = b.count[0];
+    const int n = min(b.count[0], b.nframes);
     const int nw = c.W > 128 ? 3 : 2, pad = 64 * nw - c.W;
     uint32_t mk[H];
 #pragma unroll
@@ -840,7 +842,10 @@ int bch_enqueue(drx_bch* b, uint8_t* cw, size_t stride, int32_t* result, int nfr
         k_bch_correct<16><<<grid, kFixThreads, 0, s>>>(p);
     else
         k_bch_correct<14><<<grid, kFixThreads, 0, s>>>(p);
-    return cuda_check(cudaGetLastError(), "BCH correction") ? 0 : -1;
+    if (cuda_check(cudaGetLastError(), "BCH correction"))
+        return 0;
+    cudaMemsetAsync(b->count, 0, 2 * sizeof(int), s); /* the queue that nothing will read */
+    return -1;
 }
 
 }  // namespace
