@@ -40,6 +40,9 @@ namespace {
  * batch of 21 codes (49 CTAs each) took 9.93 ms, with eight 9.49, with sixteen
  * 8.73 and with 24 8.83; at 16384 frames 56.2, 54.6, 54.4 and 55.3 ms. */
 constexpr int kSideStreams = 16;
+/* Each branch has its own message slabs (up to 76 MB); where the device has no
+ * room for all of them, four branches do. */
+constexpr int kFewBranches = 4;
 
 }  // namespace
 
@@ -307,7 +310,6 @@ int plan_mix(drx_ldpc_mix* m, int nframes, const int32_t* code, const int8_t* ll
     std::vector<int> code_side(ncodes, 0);
     std::vector<int> code_grid(ncodes, 0);
     std::vector<size_t> code_slab(ncodes, 0);
-    int k = 0;
     for (int c : corder) {
         if (!count[c])
             continue;
@@ -316,15 +318,28 @@ int plan_mix(drx_ldpc_mix* m, int nframes, const int32_t* code, const int8_t* ll
         code_slab[c] = pair ? decode_pair_msg_bytes(h->code.R, h->pair_kid) : decode_msg_bytes(h->code.R, h->code.dclass);
         code_grid[c] = pair ? std::min((count[c] + 1) / 2, h->pair_ctas_per_sm * h->sms)
                             : std::min(count[c], h->ctas_per_sm * h->sms);
-        code_side[c] = k;
-        side_bytes[k] = std::max(side_bytes[k], code_slab[c] * (size_t)code_grid[c]);
-        k = (k + 1) % kSideStreams;
     }
-    size_t total = 0;
-    for (int s = 0; s < kSideStreams; s++) {
-        side_off[s] = total;
-        total += (side_bytes[s] + 255) & ~(size_t)255;
-    }
+    auto assign_branches = [&](int branches) {
+        std::fill(side_bytes.begin(), side_bytes.end(), 0);
+        int k = 0;
+        for (int c : corder) {
+            if (!count[c])
+                continue;
+            code_side[c] = k;
+            side_bytes[k] = std::max(side_bytes[k], code_slab[c] * (size_t)code_grid[c]);
+            k = (k + 1) % branches;
+        }
+        size_t bytes = 0;
+        for (int s = 0; s < kSideStreams; s++) {
+            side_off[s] = bytes;
+            bytes += (side_bytes[s] + 255) & ~(size_t)255;
+        }
+        return bytes;
+    };
+    size_t total = assign_branches(kSideStreams);
+    size_t mem_free = 0, mem_all = 0;
+    if (cudaMemGetInfo(&mem_free, &mem_all) == cudaSuccess && total > mem_free / 2)
+        total = assign_branches(kFewBranches);
     const size_t mix_slab = decode_msg_bytes(
         std::max_element(m->codes.begin(), m->codes.end(), [](drx_ldpc* a, drx_ldpc* b) { return a->code.R < b->code.R; })[0]->code.R,
         m->dclass_max);
