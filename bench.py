@@ -598,7 +598,7 @@ def run_b200(args):
                         "reads scaled by this launch's frames and writes (L2 write-backs of the per-CTA "
                         "message slab) by its frame-iterations; against the HBM algorithmic bytes below",
         "issue": {"issue_active_pct": prof.get("issue_pct"), "alu_pipe_pct": prof.get("alu_pct"),
-                  "note": "ncu on the profiled small case: integer issue on the ALU pipe binds"},
+                  "note": "ncu on the profiled small case: instruction issue and barrier waits bind"},
         "hbm": {"achieved": hbm_bytes / kern_s / 1e9, "peak": hbm_peak,
                 "frac": hbm_bytes / kern_s / 1e9 / hbm_peak, "unit": "GB/s",
                 "peak_source": "measured (MEASURED_PEAKS.json hbm_gbs)" if "hbm_gbs" in peaks else "fallback",
