@@ -307,12 +307,12 @@ __global__ void __launch_bounds__(256) k_demap(const __grid_constant__ DemapPara
 
 /* The same for rows that are all aligned and whole: symbols on 16 bytes, LLRs on
  * 8, symbol groups of four without a remainder, no padded label bits.  No row is
- * looked at for its alignment and no store for its end, and the pointers step.
- * Bound by instruction issue, 225 for four 8PSK symbols of which 186 are the
- * distances, minimums and roundings (287 in the general kernel): 4096 normal
- * 8PSK frames 0.218 ms, 68 % of the measured HBM rate; 0.241 in the general
+ * looked at for its alignment and no store for its end, and the pointers step:
+ * 225 instructions for four 8PSK symbols, of which 186 are the distances,
+ * minimums and roundings (287 in the general kernel).  4096 normal 8PSK frames
+ * back to back 0.182 ms, 82 % of the measured HBM rate, which now binds; 0.241 in the general
  * kernel as it was, 0.227 with the minimums from a tree and the rounding by an
- * addition. */
+ * addition, 0.217 in this kernel with eight blocks per SM. */
 template <int BITS>
 __global__ void __launch_bounds__(256) k_demap_rows(const __grid_constant__ DemapParams p)
 {
@@ -390,7 +390,14 @@ cudaError_t launch_bits(const DemapParams& p, dim3 grid, cudaStream_t s)
 cudaError_t launch_demap(const DemapParams& p, int sms, cudaStream_t s)
 {
     const int gx = (((p.nsym + 3) / 4) + 255) / 256;
-    const int gy = std::max(1, std::min(p.nframes, std::max(1, 8 * sms / gx)));
+    /* 32 blocks per SM, of which five are resident (8PSK): a row of blocks takes a
+     * few tens of frames, so the last ones leave no SM idle for long.  4096 normal
+     * frames at 8, 16, 32 and 64 blocks per SM: 8PSK 0.217, 0.191, 0.182, 0.179 ms,
+     * QPSK 0.240, 0.216, 0.215, 0.209, 32APSK 0.317, 0.316, 0.319, 0.323; 512 8PSK
+     * frames 28.0, 27.0, 27.1, 29.3 us.  (Five, one wave: 0.204 ms for 8PSK, 0.217
+     * for QPSK.)  Two symbols' sums and products in one packed FP32 instruction gave
+     * 0.185 ms for 8PSK and 0.347 for 32APSK (more registers). */
+    const int gy = std::max(1, std::min(p.nframes, std::max(1, 32 * sms / gx)));
     const dim3 grid(gx, std::min(gy, 65535));
     switch (p.qpsk ? 2 : p.bits) {
     case 2: return launch_bits<2>(p, grid, s);
