@@ -254,13 +254,19 @@ int enqueue(drx_ldpc* d, const int8_t* llr, size_t llr_stride, uint8_t* out, siz
         grid = std::min((nframes + 1) / 2, d->pair_ctas_per_sm * d->sms);
         p.group = 0;
         p.work = work;
-        if (!cuda_ok(cudaMemsetAsync(work, 0, sizeof(unsigned), s), "cudaMemsetAsync"))
+        const bool own = !(x && (x->msg || x->work));
+        if (!cuda_ok(cudaMemsetAsync(work, 0, (own ? 2 : 1) * sizeof(unsigned), s), "cudaMemsetAsync"))
             return -1;
         const size_t slab = decode_pair_msg_bytes(d->code.R, d->pair_kid);
-        if (!(x && x->msg) && !ensure_scratch(d, slab * (size_t)grid))
+        if (!(x && x->msg) && !ensure_scratch(d, kOrderBytes + slab * (size_t)grid))
             return -1;
-        p.msg = x && x->msg ? x->msg : d->msg;
+        p.msg = x && x->msg ? x->msg : (char*)d->msg + kOrderBytes;
         p.msg_stride = slab;
+        if (own && !p.rows && !p.nframes_dev && order_frames(d->code.N, nframes, 2 * grid, max_iter)) {
+            if (!cuda_ok(launch_order(llr, llr_stride, d->code.N, nframes, d->msg, work + 1, d->sms, s), "frame order"))
+                return -1;
+            p.rows = (const int32_t*)d->msg;
+        }
         return cuda_ok(launch_decode_pair(p, d->pair_kid, d->pair_smem, grid, s), "decoder launch") ? 0 : -1;
     }
     const int pair_capacity = d->pair_ctas_per_sm * d->sms;
