@@ -141,6 +141,12 @@ def load_learned_table():
     return T.load_table(SHORT, RATE, CONST, LEARNED_ITERS)
 
 
+def order_launches(nframes, nsm):
+    """1 if a batch of normal 3/5 frames is put in order first (more frames
+    than the decoder's lanes, two CTAs of two per SM), else 0."""
+    return 1 if 4 * nsm < nframes <= 16384 else 0
+
+
 def profiled_figures():
     """Figures of the committed ncu summary of the decode kernel: DRAM bytes
     read per frame and written per frame-iteration, issue and ALU-pipe
@@ -690,12 +696,13 @@ def run_b200(args):
                 "fallback_frac": float(fb_all.mean()),
                 "avg_iterations_learned_pass": float(torch.stack(l_it).float()[fb_all == 0].mean())
                 if bool((fb_all == 0).any()) else None,
-                "plain_fallback_max_iter": fallback_iters, "launches_per_step": 3,
+                "plain_fallback_max_iter": fallback_iters,
+                "launches_per_step": 3 + order_launches(F, nsm),
                 "decoder": "learned scaled/offset min-sum at int8 (Q8 table per iteration and degree class), "
                            "frames failing the syndrome re-decoded by the plain decoder on the device"})
         else:
             res.update({
-                "launches_per_step": 1,
+                "launches_per_step": 1 + order_launches(F, nsm),
                 "decoder": "learned scaled/offset min-sum at int8 (Q8 table per iteration and degree class), "
                            "one pass of at most %d iterations with per-frame stopping, no plain decoder" % L})
         return res
@@ -780,7 +787,7 @@ def run_b200(args):
             "dropin": dropin,
             "learned": learned, "learned_30it_one_pass": learned30,
             "mixed_modcod": mix_res, "mixed_modcod_learned": mix_learned, "bch": bch, "demapper": demap,
-            "gpu_launches": args.steps,
+            "gpu_launches": args.steps * (1 + order_launches(F, nsm)),
         }
         print(json.dumps(line))
     if world > 1:
