@@ -105,6 +105,8 @@ __device__ __forceinline__ void demap_symbol(const DemapParams& p, float x, floa
         out[1] = quantise8(__fmul_rn(kq, y));
         return;
     }
+    /* from infinity: a bit value whose distances are all NaN (infinite symbols)
+     * has no nearest point, and the other value wins */
     float m0[BITS], m1[BITS];
 #pragma unroll
     for (int b = 0; b < BITS; b++)
@@ -188,8 +190,8 @@ __device__ __forceinline__ void demap_symbol(const DemapParams& p, float x, floa
         bit_minima<BITS>(v, lo, hi);
 #pragma unroll
         for (int L = 0; L < BITS; L++) {
-            m0[BITS - 1 - L] = lo[L];
-            m1[BITS - 1 - L] = hi[L];
+            m0[BITS - 1 - L] = fminf(m0[BITS - 1 - L], lo[L]);
+            m1[BITS - 1 - L] = fminf(m1[BITS - 1 - L], hi[L]);
         }
     }
 #pragma unroll
