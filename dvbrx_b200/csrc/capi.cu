@@ -91,6 +91,10 @@ bool ensure_stage(drx_ldpc* d, size_t nframes)
     return true;
 }
 
+/* Message scratch of at least `need` bytes (a multiple of 16).  The frame order
+ * of a per-frame batch follows it in the same allocation, whoever asked for it,
+ * so that a call which orders its frames needs no more than any other that
+ * fills as many CTAs (and a captured one allocates nothing after it). */
 bool ensure_scratch(drx_ldpc* d, size_t need)
 {
     if (d->msg_cap >= need)
@@ -99,7 +103,7 @@ bool ensure_scratch(drx_ldpc* d, size_t need)
     cudaFree(d->msg);
     d->msg = nullptr;
     d->msg_cap = 0;
-    if (!cuda_ok(drxg::dev_malloc(&d->msg, need), "cudaMalloc(messages)"))
+    if (!cuda_ok(drxg::dev_malloc(&d->msg, need + kOrderBytes), "cudaMalloc(messages)"))
         return false;
     d->msg_cap = need;
     return true;
@@ -116,17 +120,7 @@ bool use_pair(const drx_ldpc* d)
 
 bool ensure_msg(drx_ldpc* d, int grid)
 {
-    const size_t need = decode_msg_bytes(d->code.R, d->code.dclass) * (size_t)grid;
-    if (d->msg_cap >= need)
-        return true;
-    cudaStreamSynchronize(d->stream);
-    cudaFree(d->msg);
-    d->msg = nullptr;
-    d->msg_cap = 0;
-    if (!cuda_ok(drxg::dev_malloc(&d->msg, need), "cudaMalloc(messages)"))
-        return false;
-    d->msg_cap = need;
-    return true;
+    return ensure_scratch(d, decode_msg_bytes(d->code.R, d->code.dclass) * (size_t)grid);
 }
 
 bool ensure_sync(drx_ldpc* d, size_t words)
@@ -258,14 +252,15 @@ int enqueue(drx_ldpc* d, const int8_t* llr, size_t llr_stride, uint8_t* out, siz
         if (!cuda_ok(cudaMemsetAsync(work, 0, (own ? 2 : 1) * sizeof(unsigned), s), "cudaMemsetAsync"))
             return -1;
         const size_t slab = decode_pair_msg_bytes(d->code.R, d->pair_kid);
-        if (!(x && x->msg) && !ensure_scratch(d, kOrderBytes + slab * (size_t)grid))
+        if (!(x && x->msg) && !ensure_scratch(d, slab * (size_t)grid))
             return -1;
-        p.msg = x && x->msg ? x->msg : (char*)d->msg + kOrderBytes;
+        p.msg = x && x->msg ? x->msg : d->msg;
         p.msg_stride = slab;
         if (own && !p.rows && !p.nframes_dev && order_frames(d->code.N, nframes, 2 * grid, max_iter)) {
-            if (!cuda_ok(launch_order(llr, llr_stride, d->code.N, nframes, d->msg, work + 1, d->sms, s), "frame order"))
+            void* order = (char*)d->msg + d->msg_cap;
+            if (!cuda_ok(launch_order(llr, llr_stride, d->code.N, nframes, order, work + 1, d->sms, s), "frame order"))
                 return -1;
-            p.rows = (const int32_t*)d->msg;
+            p.rows = (const int32_t*)order;
         }
         return cuda_ok(launch_decode_pair(p, d->pair_kid, d->pair_smem, grid, s), "decoder launch") ? 0 : -1;
     }

@@ -36,7 +36,7 @@ struct drx_ldpc {
     int test_skip_vote = 0; /* testing: CTA test_skip_vote - 1 of group launches never votes */
     cudaStream_t stream = nullptr;
     /* scratch */
-    void* msg = nullptr;
+    void* msg = nullptr; /* msg_cap bytes of messages, then a frame order (kOrderBytes) */
     size_t msg_cap = 0;
     unsigned* work = nullptr;
     unsigned* sync = nullptr;

@@ -161,8 +161,8 @@ size_t decode_pair_msg_bytes(int R, int kid);
 int decode_pair_ctas_per_sm(int kid, size_t smem);
 cudaError_t launch_decode_pair(const DecodeParams& p, int kid, size_t smem, int grid, cudaStream_t stream);
 
-/* Processing order of a per-frame batch (order.cu): weakest LLRs first, at the
- * head of `scratch` (kOrderBytes); *ticket zero before. */
+/* Processing order of a per-frame batch (order.cu): weakest LLRs first, in the
+ * first nframes words of `scratch` (kOrderBytes); *ticket zero before. */
 constexpr int kOrderFrames = 16384;
 constexpr size_t kOrderBytes = 2 * sizeof(int32_t) * kOrderFrames;
 cudaError_t launch_order(const int8_t* llr, size_t stride, int N, int n, void* scratch, unsigned* ticket, int sms,
