@@ -150,6 +150,8 @@ def lib():
         L.drx_bch_decode.restype = ip
         L.drx_bch_decode_device.argtypes = [vp, vp, sz, vp, ip, vp]
         L.drx_bch_decode_device.restype = ip
+        L.drx_bch_test_left_over.argtypes = [vp, ip]
+        L.drx_bch_test_left_over.restype = ip
         L.drx_bch_encode_device.argtypes = [vp, vp, sz, ip, vp]
         L.drx_bch_encode_device.restype = ip
         L.drx_ldpc_mix_set_learned.argtypes = [vp, ip, ip, ip, vp, vp, vp]
@@ -497,6 +499,12 @@ class Bch:
         if r != 0:
             raise RuntimeError("drx_bch_decode_device: " + last_error())
         return result
+
+    def test_left_over(self, frames):
+        """``drx_bch_test_left_over`` (testing): `frames` queued frames stay
+        behind in the workspace, as after a decode that was cut short."""
+        if self._lib.drx_bch_test_left_over(self.h, int(frames)) != 0:
+            raise RuntimeError("drx_bch_test_left_over: " + last_error())
 
 
 TILING_ONE_LAUNCH, TILING_PER_CODE, TILING_ONE_LAUNCH_PAIR = 1, 2, 3  # DRX_TILING_*

@@ -61,7 +61,7 @@ struct BchBatch {
     int nframes;
     unsigned long long* rem; /* per frame: its remainder, where it is not zero */
     int32_t* queue;          /* frames with a remainder */
-    int* count;              /* queue length, CTAs of the correction kernel that are done */
+    int* count;              /* queue length, zeroed before the remainder kernel */
 };
 
 /*
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(32 * kRemMaxWarps) k_bch_remainder(BchBatch b,
                 for (int w = 0; w < NW; w++)
                     b.rem[(size_t)f * NW + w] = r[w];
                 const int at = atomicAdd(b.count, 1);
-                if (at < b.nframes) /* always, unless an earlier batch's correction never ran */
+                if (at < b.nframes) /* always, unless another call on the handle overlaps */
                     b.queue[at] = f;
             }
         }
@@ -442,10 +442,11 @@ __global__ void __launch_bounds__(kFixThreads, 4) k_bch_correct(BchBatch b)
     for (int q0 = blockIdx.x; q0 < n; q0 += kFixWarps * gridDim.x) {
         /* each warp finds one frame's locator */
         const int qi = q0 + warp * gridDim.x;
+        int f = qi < n ? b.queue[qi] : -1;
+        f = f < b.nframes ? f : -1; /* a row of another batch, if calls on the handle overlap */
         if (lane == 0)
-            s.frame[warp] = qi < n ? b.queue[qi] : -1;
-        if (qi < n) {
-            const int f = b.queue[qi];
+            s.frame[warp] = f;
+        if (f >= 0) {
             /* S_1, S_3 ..: two in a word */
             uint32_t so[6] = { 0, 0, 0, 0, 0, 0 };
 #pragma unroll
@@ -606,14 +607,6 @@ __global__ void __launch_bounds__(kFixThreads, 4) k_bch_correct(BchBatch b)
             __syncthreads();
         }
         __syncthreads();
-    }
-    /* the last CTA empties the queue for the next batch */
-    if (t == 0) {
-        __threadfence();
-        if (atomicAdd(b.count + 1, 1) == (int)gridDim.x - 1) {
-            b.count[0] = 0;
-            b.count[1] = 0;
-        }
     }
 }
 
@@ -835,17 +828,16 @@ int bch_enqueue(drx_bch* b, uint8_t* cw, size_t stride, int32_t* result, int nfr
     p.rem = b->rem;
     p.queue = b->queue;
     p.count = b->count;
-    if (!cuda_check(remainders<false>(b, p, b->nbch / 8, s), "BCH remainder"))
+    /* in every call: a length left by one that failed or overlapped another ends with it */
+    if (!cuda_check(cudaMemsetAsync(b->count, 0, sizeof(int), s), "cudaMemsetAsync") ||
+        !cuda_check(remainders<false>(b, p, b->nbch / 8, s), "BCH remainder"))
         return -1;
     const int grid = std::min(nframes, 4 * b->sms);
     if (b->m == 16)
         k_bch_correct<16><<<grid, kFixThreads, 0, s>>>(p);
     else
         k_bch_correct<14><<<grid, kFixThreads, 0, s>>>(p);
-    if (cuda_check(cudaGetLastError(), "BCH correction"))
-        return 0;
-    cudaMemsetAsync(b->count, 0, 2 * sizeof(int), s); /* the queue that nothing will read */
-    return -1;
+    return cuda_check(cudaGetLastError(), "BCH correction") ? 0 : -1;
 }
 
 }  // namespace
@@ -880,8 +872,7 @@ drx_bch* drx_bch_new(const drx_fec_params* p)
     const size_t o_syn = tab.size() * 8, o_sets = o_syn + syn.size() * 4, o_anf = o_sets + sets.size() * 4,
                  o_lg = o_anf + anf.size() * 2, total = o_lg + lg.size() * 2 + 64;
     ok = ok && cuda_check(drxg::dev_malloc(&b->blob, total), "cudaMalloc(bch tables)") &&
-         cuda_check(drxg::dev_malloc(&b->count, 2 * sizeof(int)), "cudaMalloc") &&
-         cuda_check(cudaMemset(b->count, 0, 2 * sizeof(int)), "cudaMemset") &&
+         cuda_check(drxg::dev_malloc(&b->count, sizeof(int)), "cudaMalloc") &&
          cuda_check(drxg::dev_malloc(&b->d_cw, (size_t)b->nbch / 8), "cudaMalloc") &&
          cuda_check(drxg::dev_malloc(&b->d_res, sizeof(int32_t)), "cudaMalloc");
     if (ok) {
@@ -954,6 +945,15 @@ int drx_bch_encode_device(drx_bch* b, uint8_t* cw, size_t stride, int nframes, v
     return cuda_check(remainders<true>(b, p, b->kbch / 8, stream ? (cudaStream_t)stream : b->stream), "BCH encode")
                ? 0
                : -1;
+}
+
+int drx_bch_test_left_over(drx_bch* b, int frames)
+{
+    if (!b || frames < 0) {
+        set_error("drx_bch_test_left_over: NULL handle or a negative count");
+        return -1;
+    }
+    return cuda_check(cudaMemcpy(b->count, &frames, sizeof(int), cudaMemcpyHostToDevice), "cudaMemcpy") ? 0 : -1;
 }
 
 int drx_bch_decode(drx_bch* b, uint8_t* cw)

@@ -330,9 +330,15 @@ int drx_bch_decode(drx_bch* b, uint8_t* cw);
 /* No counterpart in the reference (its decoder takes one word per call).
  * Decode nframes device-resident codewords in place (row f at cw + f *
  * stride) asynchronously on `stream`, straight after the LDPC decode of the
- * same rows: result[f] (device) receives what drx_bch_decode returns.
- * Returns 0 if the work was queued. */
+ * same rows: result[f] (device) receives what drx_bch_decode returns.  Calls
+ * on one handle share its workspace and must not overlap: on another stream, a
+ * call waits (an event) for the one before.  Returns 0 if the work was queued. */
 int drx_bch_decode_device(drx_bch* b, uint8_t* cw, size_t stride, int32_t* result, int nframes, void* stream);
+
+/* Testing hook: leaves `frames` queued frames behind in the handle's
+ * workspace, as a decode that was cut short would.  Later decodes must not
+ * see them.  Returns 0, or -1. */
+int drx_bch_test_left_over(drx_bch* b, int frames);
 
 /* No counterpart in the reference (the transmitter side, for test and
  * benchmark frames): encode nframes device rows in place, the kbch message
