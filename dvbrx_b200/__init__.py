@@ -150,6 +150,8 @@ def lib():
         L.drx_bch_decode.restype = ip
         L.drx_bch_decode_device.argtypes = [vp, vp, sz, vp, ip, vp]
         L.drx_bch_decode_device.restype = ip
+        L.drx_ldpc_mix_branches.argtypes = [vp]
+        L.drx_ldpc_mix_branches.restype = ip
         L.drx_bch_test_left_over.argtypes = [vp, ip]
         L.drx_bch_test_left_over.restype = ip
         L.drx_bch_encode_device.argtypes = [vp, vp, sz, ip, vp]
@@ -595,6 +597,10 @@ class LdpcMix:
         plan lacks it)."""
         v = self._lib.drx_ldpc_mix_tuned_ms(self.h, int(tiling))
         return None if v < 0 else v
+
+    def branches(self):
+        """``drx_ldpc_mix_branches``: branches of the plan's per-code graph."""
+        return self._lib.drx_ldpc_mix_branches(self.h)
 
     def tune(self, stream=None):
         """Times every tiling of the plan on the planned batch; returns

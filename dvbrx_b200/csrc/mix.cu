@@ -40,8 +40,8 @@ namespace {
  * batch of 21 codes (49 CTAs each) took 9.93 ms, with eight 9.49, with sixteen
  * 8.73 and with 24 8.83; at 16384 frames 56.2, 54.6, 54.4 and 55.3 ms. */
 constexpr int kSideStreams = 16;
-/* Each branch has its own message slabs (up to 76 MB); where the device has no
- * room for all of them, four branches do. */
+/* Each branch has its own message slabs (up to 76 MB); where they would take more
+ * than half of the free device memory, or cannot be had, four branches do. */
 constexpr int kFewBranches = 4;
 
 }  // namespace
@@ -58,6 +58,7 @@ struct drx_ldpc_mix {
     cudaEvent_t fork = nullptr, join[kSideStreams] = {};
     /* plan */
     int nframes = 0;
+    int branches = 0; /* of the per-code graph, at most */
     int32_t* d_frame_code = nullptr;
     int32_t* d_order = nullptr;
     unsigned* d_work = nullptr; /* one counter per code, then one for the one-launch kernel */
@@ -109,6 +110,7 @@ void release_plan(drx_ldpc_mix* m)
     m->d_work = nullptr;
     m->d_msg = nullptr;
     m->nframes = 0;
+    m->branches = 0;
 }
 
 bool pair_runs(const drx_ldpc* h) { return h->variant != DRX_VARIANT_FRAME && h->pair_ctas_per_sm > 0; }
@@ -336,15 +338,16 @@ int plan_mix(drx_ldpc_mix* m, int nframes, const int32_t* code, const int8_t* ll
         }
         return bytes;
     };
-    size_t total = assign_branches(kSideStreams);
+    int branches = kSideStreams;
+    size_t side_total = assign_branches(branches);
     size_t mem_free = 0, mem_all = 0;
-    if (cudaMemGetInfo(&mem_free, &mem_all) == cudaSuccess && total > mem_free / 2)
-        total = assign_branches(kFewBranches);
+    if (cudaMemGetInfo(&mem_free, &mem_all) == cudaSuccess && side_total > mem_free / 2)
+        side_total = assign_branches(branches = kFewBranches);
     const size_t mix_slab = decode_msg_bytes(
         std::max_element(m->codes.begin(), m->codes.end(), [](drx_ldpc* a, drx_ldpc* b) { return a->code.R < b->code.R; })[0]->code.R,
         m->dclass_max);
     const int mix_grid = std::min(nframes, m->mix_ctas * m->sms);
-    total = std::max(total, mix_slab * (size_t)mix_grid);
+    size_t launch_total = mix_slab * (size_t)mix_grid; /* of the one-launch kernels */
 
     /* one launch, two frames per CTA (plain plans, every code of the batch
      * with a shape in the mixed kernel): shared memory and slab of the
@@ -394,12 +397,21 @@ int plan_mix(drx_ldpc_mix* m, int nframes, const int32_t* code, const int8_t* ll
             }
             pair_host[4 * (size_t)ncodes + k] = corder[std::min(ci, ncodes - 1)];
         }
-        total = std::max(total, pair_slab * (size_t)pair_grid);
+        launch_total = std::max(launch_total, pair_slab * (size_t)pair_grid);
     }
+    auto alloc_messages = [&]() {
+        cudaError_t e = drxg::dev_malloc(&m->d_msg, std::max(side_total, launch_total));
+        if (e == cudaErrorMemoryAllocation && branches > kFewBranches) {
+            cudaGetLastError(); /* not the plan's failure yet */
+            side_total = assign_branches(branches = kFewBranches);
+            e = drxg::dev_malloc(&m->d_msg, std::max(side_total, launch_total));
+        }
+        return e;
+    };
     if (!cuda_check(drxg::dev_malloc(&m->d_frame_code, sizeof(int32_t) * nframes), "cudaMalloc") ||
         !cuda_check(drxg::dev_malloc(&m->d_order, sizeof(int32_t) * nframes), "cudaMalloc") ||
         !cuda_check(drxg::dev_malloc(&m->d_work, sizeof(unsigned) * (2 * ncodes + 1)), "cudaMalloc") ||
-        !cuda_check(drxg::dev_malloc(&m->d_msg, total), "cudaMalloc") ||
+        !cuda_check(alloc_messages(), "cudaMalloc(messages)") ||
         !cuda_check(cudaMemcpy(m->d_frame_code, code, sizeof(int32_t) * nframes, cudaMemcpyHostToDevice), "cudaMemcpy") ||
         !cuda_check(cudaMemcpy(m->d_order, order.data(), sizeof(int32_t) * nframes, cudaMemcpyHostToDevice), "cudaMemcpy") ||
         (pair_plan &&
@@ -437,6 +449,7 @@ int plan_mix(drx_ldpc_mix* m, int nframes, const int32_t* code, const int8_t* ll
             ok = m->d_fb_ok;
     }
     m->nframes = nframes;
+    m->branches = branches;
     /* kernel attributes are set before capture (not a stream operation) */
     decode_mix_ctas_per_sm(m->dclass_max, m->mix_smem);
     if (pair_plan)
@@ -654,6 +667,8 @@ int drx_ldpc_mix_set_tiling(drx_ldpc_mix* m, int tiling)
     m->tiling = tiling;
     return tiling;
 }
+
+int drx_ldpc_mix_branches(const drx_ldpc_mix* m) { return m ? m->branches : -1; }
 
 int drx_ldpc_mix_run(drx_ldpc_mix* m, void* stream)
 {

@@ -232,6 +232,11 @@ int drx_ldpc_mix_tune(drx_ldpc_mix* m, void* stream, float* ms_one_launch, float
 /* The autotuner's time of a tiling in ms, -1 if the plan lacks it. */
 float drx_ldpc_mix_tuned_ms(const drx_ldpc_mix* m, int tiling);
 
+/* Most codes that the plan's per-code graph decodes at once (its branches, each
+ * with its own message memory): 16, or 4 where device memory is short; 0 without
+ * a plan, -1 for NULL. */
+int drx_ldpc_mix_branches(const drx_ldpc_mix* m);
+
 /* Launch the plan's graph (the tuned or set tiling) on `stream`. */
 int drx_ldpc_mix_run(drx_ldpc_mix* m, void* stream);
 
