@@ -434,7 +434,7 @@ __global__ void __launch_bounds__(kFixThreads, 4) k_bch_correct(BchBatch b)
     const BchDev& c = b.c;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int n = min(b.count[0], b.nframes);
-    const int nw = c.W > 128 ? 3 : 2, pad = 64 * nw - c.W;
+    const int nw = c.W > 128 ? 3 : 2;
     uint32_t mk[H];
 #pragma unroll
     for (int h = 0; h < H; h++)

@@ -636,7 +636,7 @@ drx_ldpc* drx_ldpc_new(const drx_fec_params* p, const char* rate)
     if (d->pair_kid >= 0) {
         auto smem_of = [&](int kid) {
             return decode_pair_smem_bytes(d->code.N, d->code.K, (int)d->code.ent.size() / 2,
-                                          (int)d->code.steps.size(), d->code.q, kid);
+                                          d->code.q, kid);
         };
         d->pair_smem = smem_of(d->pair_kid);
         d->pair_ctas_per_sm = decode_pair_ctas_per_sm(d->pair_kid, d->pair_smem);

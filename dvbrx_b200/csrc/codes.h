@@ -68,9 +68,6 @@ struct Code {
  * the codes it runs. */
 constexpr int kNumClasses = 6;
 constexpr int kClassDeg[kNumClasses] = { 7, 11, 14, 18, 22, 32 };
-/* smallest information-link count of a layer in the codes of each class
- * (the frame-pair kernel instantiates link counts kClassCntLo .. max) */
-constexpr int kClassCntLo[kNumClasses] = { 1, 5, 7, 12, 14, 25 };
 int degree_class(int deg_max);
 
 /* Rate string -> table index (cg_rates_normal / cg_rates_short), or -1.

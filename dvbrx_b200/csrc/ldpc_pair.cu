@@ -65,12 +65,12 @@ static const std::vector<PairKernel>& kernels()
 
 /* Dynamic shared memory of a pair kernel for a code: the posterior words
  * (every bit, or the information bits of a parity-out kernel and the last
- * parity layer), the link table, layer offsets and level steps */
-size_t decode_pair_smem_bytes(int N, int K, int nent, int nsteps, int q, int kid)
+ * parity layer), the link table and layer offsets */
+size_t decode_pair_smem_bytes(int N, int K, int nent, int q, int kid)
 {
     const bool po = kid >= 0 && kid < (int)kernels().size() && kernels()[kid].pm == 2;
     return a16h(2 * (size_t)(po ? K : N)) + (po ? a16h(2 * (size_t)kQCp) : 0) + a16h(sizeof(int2) * nent) +
-           a16h(sizeof(uint16_t) * (q + 1)) + a16h(sizeof(uint32_t) * nsteps);
+           a16h(sizeof(uint16_t) * (q + 1));
 }
 
 /* message slab of one CTA: one record per check, 8 or 16 bytes; a

@@ -247,7 +247,7 @@ struct PairCheck {
     }
 
     template <bool LEV>
-    __device__ __forceinline__ void read_all(const uint16_t* __restrict__ post, uint32_t r0, uint32_t r1)
+    __device__ __forceinline__ void read_all(uint32_t r0, uint32_t r1)
     {
         const uint32_t shared = inm | outm;
         auto slot = [&](int k) {
@@ -307,8 +307,7 @@ struct PairCheck {
         recw = h_to_int(h_min(m0, kH32)) | (h_to_int(h_min(m1, kH32)) << 6);
     }
 
-    __device__ __forceinline__ void write_rest(uint16_t* __restrict__ post, Rec* __restrict__ dst, uint32_t& o0,
-                                               uint32_t& o1)
+    __device__ __forceinline__ void write_rest(Rec* __restrict__ dst, uint32_t& o0, uint32_t& o1)
     {
         const uint32_t wm = live & ~outm;
         uint32_t nsg = 0, nsg1 = 0;
@@ -380,7 +379,6 @@ struct PairFrame {
     uint16_t* post;
     const int2* ent; /* (shared byte address of the link group's first word, -2 a) */
     const uint16_t* eoff;
-    const uint32_t* steps;
     /* parity out of shared memory (PO kernels): the posterior word of
      * parity bit (i, j) is gpar[360 i + j] (global, this CTA's slab) for
      * i < q - 1 and wrap[j] (shared) for the last layer */
@@ -405,8 +403,6 @@ __device__ PairFrame stage_pair(const DevCode& c, char* smem, uint16_t* gpar)
     int2* ent = (int2*)(smem + off);
     off += a16p(sizeof(int2) * c.nent);
     uint16_t* eoff = (uint16_t*)(smem + off);
-    off += a16p(sizeof(uint16_t) * (c.q + 1));
-    uint32_t* steps = (uint32_t*)(smem + off);
     /* entries (360 g - a, a) as (shared byte address of group g's first
      * posterior word, -2 a): the link of check j is word (j - a) mod 360 of
      * the group, at byte offset min(u, u + 720), u = 2 j - 2 a unsigned */
@@ -417,11 +413,8 @@ __device__ PairFrame stage_pair(const DevCode& c, char* smem, uint16_t* gpar)
     }
     for (int k = threadIdx.x; k <= c.q; k += blockDim.x)
         eoff[k] = c.eoff[k];
-    for (int k = threadIdx.x; k < c.nsteps; k += blockDim.x)
-        steps[k] = c.steps[k];
     f.ent = ent;
     f.eoff = eoff;
-    f.steps = steps;
     return f;
 }
 
@@ -724,8 +717,8 @@ __device__ __forceinline__ void level_step(Ck& ck, uint32_t inner, bool mine, bo
 template <int DM, int LS, bool WIDE, bool LEARNED, bool PO>
 __device__ __forceinline__ void layer_pair(const PairFrame& fr, const DevCode& c, const int2* ent, int i, int nlev,
                                            PairRec<WIDE> rec, unsigned long long meta, uint32_t fresh,
-                                           PairRec<WIDE>* __restrict__ msg, int lA, int lB, uint32_t r0,
-                                           uint32_t r1, uint32_t& o0, uint32_t& o1)
+                                           PairRec<WIDE>* __restrict__ msg, uint32_t r0, uint32_t r1,
+                                           uint32_t& o0, uint32_t& o1)
 {
     const int t = threadIdx.x;
     const bool active = t < kQCp;
@@ -740,9 +733,9 @@ __device__ __forceinline__ void layer_pair(const PairFrame& fr, const DevCode& c
         ck.setup(ent, c.K, c.q, i, j, rec, fresh, meta,
                  (uint32_t)__cvta_generic_to_shared(fr.post));
         if (LS > 0 && nlev > 1)
-            ck.template read_all<true>(fr.post, r0, r1);
+            ck.template read_all<true>(r0, r1);
         else
-            ck.template read_all<false>(fr.post, r0, r1);
+            ck.template read_all<false>(r0, r1);
     } else {
         ck.idle((uint32_t)__cvta_generic_to_shared(fr.post));
     }
@@ -788,7 +781,7 @@ __device__ __forceinline__ void layer_pair(const PairFrame& fr, const DevCode& c
     }
     if (active) {
         ck.finish(LEARNED, lp);
-        ck.write_rest(fr.post, msg + kQCp * i + j, o0, o1);
+        ck.write_rest(msg + kQCp * i + j, o0, o1);
     }
     __syncthreads();
 }
@@ -797,15 +790,14 @@ __device__ __forceinline__ void layer_pair(const PairFrame& fr, const DevCode& c
 template <int A, int B, int STEP, int LS, bool WIDE, bool LEARNED, bool PO>
 __device__ __forceinline__ void layer_of_count(const PairFrame& fr, const DevCode& c, const int2* ent, int i, int cnt, int nlev,
                                                PairRec<WIDE> rec, unsigned long long meta, uint32_t fresh,
-                                               PairRec<WIDE>* __restrict__ msg, int lA, int lB, uint32_t r0,
-                                               uint32_t r1, uint32_t& o0, uint32_t& o1)
+                                               PairRec<WIDE>* __restrict__ msg, uint32_t r0, uint32_t r1,
+                                               uint32_t& o0, uint32_t& o1)
 {
     if (A == B || cnt == A)
-        layer_pair<A + 2, LS, WIDE, LEARNED, PO>(fr, c, ent, i, nlev, rec, meta, fresh, msg, lA, lB, r0, r1, o0,
-                                                       o1);
+        layer_pair<A + 2, LS, WIDE, LEARNED, PO>(fr, c, ent, i, nlev, rec, meta, fresh, msg, r0, r1, o0, o1);
     else if constexpr (A < B)
-        layer_of_count<A + STEP, B, STEP, LS, WIDE, LEARNED, PO>(fr, c, ent, i, cnt, nlev, rec, meta, fresh, msg, lA, lB,
-                                                                 r0, r1, o0, o1);
+        layer_of_count<A + STEP, B, STEP, LS, WIDE, LEARNED, PO>(fr, c, ent, i, cnt, nlev, rec, meta, fresh, msg, r0, r1,
+                                                                 o0, o1);
 }
 
 /* One decoding iteration: the layers in order; each layer's messages and
@@ -868,7 +860,7 @@ __device__ void iterate_pair(const DevCode& c, const PairFrame& fr, void* msgv, 
         const int nlev = nl;
         nl = c.nlev[i + 1 < c.q ? i + 1 : i];
         layer_of_count<A, B, EVERY ? 1 : B - A, LS, WIDE, LEARNED, PO>(fr, c, ent, i, cnt, nlev, rec, meta, fresh, msg,
-                                                                       lA, lB, r0, r1, o0, o1);
+                                                                       r0, r1, o0, o1);
         /* (i - 1, j) is final for this iteration; (i, j) goes to the next
          * layer, or, for the last layer, to the check (0, j + 1) */
         if (PO && active) {

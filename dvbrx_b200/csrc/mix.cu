@@ -367,7 +367,7 @@ int plan_mix(drx_ldpc_mix* m, int nframes, const int32_t* code, const int8_t* ll
         }
         weight[c] = (int)std::min<long long>(h->code.edges, 1 << 30);
         pair_smem = std::max(pair_smem, decode_pair_smem_bytes(h->code.N, h->code.K, (int)h->code.ent.size() / 2,
-                                                               (int)h->code.steps.size(), h->code.q, kid));
+                                                               h->code.q, kid));
         pair_slab = std::max(pair_slab, decode_pair_msg_bytes(h->code.R, kid));
     }
     int pair_grid = 0;
