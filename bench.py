@@ -141,12 +141,6 @@ def load_learned_table():
     return T.load_table(SHORT, RATE, CONST, LEARNED_ITERS)
 
 
-def order_launches(nframes, nsm):
-    """1 if a batch of normal 3/5 frames is put in order first (more frames
-    than the decoder's lanes, two CTAs of two per SM), else 0."""
-    return 1 if 4 * nsm < nframes <= 16384 else 0
-
-
 def profiled_figures():
     """Figures of the committed ncu summary of the decode kernel: DRAM bytes
     read per frame and written per frame-iteration, issue and ALU-pipe
@@ -518,7 +512,7 @@ def run_b200(args):
     p = D.fec_lookup(SHORT, RATE)
     dec = D.Ldpc(p, RATE)
     variant = dec.set_variant(D.VARIANT_FRAME if args.variant == "frame" else D.VARIANT_AUTO)
-    kernel_name = {D.VARIANT_PAIR: "drxg::k_decode_pair (two frames per CTA, 16x2 SIMD)",
+    kernel_name = {D.VARIANT_PAIR: "drxg::k_decode_pair (two frames per CTA, FP16 pairs)",
                    D.VARIANT_FRAME: "drxg::k_decode (one frame per CTA)"}[variant]
     F = args.frames
     kldpc = p.kldpc
@@ -697,12 +691,12 @@ def run_b200(args):
                 "avg_iterations_learned_pass": float(torch.stack(l_it).float()[fb_all == 0].mean())
                 if bool((fb_all == 0).any()) else None,
                 "plain_fallback_max_iter": fallback_iters,
-                "launches_per_step": 3 + order_launches(F, nsm),
+                "launches_per_step": 2 + dec.decode_launches(F, L),
                 "decoder": "learned scaled/offset min-sum at int8 (Q8 table per iteration and degree class), "
                            "frames failing the syndrome re-decoded by the plain decoder on the device"})
         else:
             res.update({
-                "launches_per_step": 1 + order_launches(F, nsm),
+                "launches_per_step": dec.decode_launches(F, L),
                 "decoder": "learned scaled/offset min-sum at int8 (Q8 table per iteration and degree class), "
                            "one pass of at most %d iterations with per-frame stopping, no plain decoder" % L})
         return res
@@ -787,7 +781,7 @@ def run_b200(args):
             "dropin": dropin,
             "learned": learned, "learned_30it_one_pass": learned30,
             "mixed_modcod": mix_res, "mixed_modcod_learned": mix_learned, "bch": bch, "demapper": demap,
-            "gpu_launches": args.steps * (1 + order_launches(F, nsm)),
+            "gpu_launches": args.steps * dec.decode_launches(F, MAX_ITER),
         }
         print(json.dumps(line))
     if world > 1:

@@ -150,6 +150,8 @@ def lib():
         L.drx_bch_decode.restype = ip
         L.drx_bch_decode_device.argtypes = [vp, vp, sz, vp, ip, vp]
         L.drx_bch_decode_device.restype = ip
+        L.drx_ldpc_decode_launches.argtypes = [vp, ip, ip, ip]
+        L.drx_ldpc_decode_launches.restype = ip
         L.drx_ldpc_mix_branches.argtypes = [vp]
         L.drx_ldpc_mix_branches.restype = ip
         L.drx_bch_test_left_over.argtypes = [vp, ip]
@@ -283,6 +285,10 @@ class Ldpc:
         if r != 0:
             raise RuntimeError("drx_ldpc_decode_device: " + last_error())
         return out, iters, ok
+
+    def decode_launches(self, nframes, max_iter, stop=STOP_FRAME):
+        """``drx_ldpc_decode_launches``: kernels of such a device batch."""
+        return self._lib.drx_ldpc_decode_launches(self.h, int(nframes), int(max_iter), int(stop))
 
     def generate(self, nframes, esn0_db, seed, constellation="QPSK", const_rate=None, llr=True,
                  info=False, llr_f16=False, stream=None):

@@ -183,6 +183,15 @@ bool upload_code(drx_ldpc* d)
     return true;
 }
 
+/* CTAs of a per-frame launch of nframes frames on the frame-pair kernel, and
+ * whether the batch is put in order before it (a call with its own scratch) */
+int pair_grid(const drx_ldpc* d, int nframes) { return std::min((nframes + 1) / 2, d->pair_ctas_per_sm * d->sms); }
+
+bool orders(const drx_ldpc* d, int nframes, int max_iter)
+{
+    return use_pair(d) && order_frames(d->code.N, nframes, 2 * pair_grid(d, nframes), max_iter);
+}
+
 /* Per-frame extras of a launch: learned check nodes, a row list and a
  * frame count read on the device (nframes is then an upper bound). */
 struct Extra {
@@ -245,7 +254,7 @@ int enqueue(drx_ldpc* d, const int8_t* llr, size_t llr_stride, uint8_t* out, siz
     int grid;
     if (stop == 0 && use_pair(d)) {
         /* two frames per CTA */
-        grid = std::min((nframes + 1) / 2, d->pair_ctas_per_sm * d->sms);
+        grid = pair_grid(d, nframes);
         p.group = 0;
         p.work = work;
         const bool own = !(x && (x->msg || x->work));
@@ -256,7 +265,7 @@ int enqueue(drx_ldpc* d, const int8_t* llr, size_t llr_stride, uint8_t* out, siz
             return -1;
         p.msg = x && x->msg ? x->msg : d->msg;
         p.msg_stride = slab;
-        if (own && !p.rows && !p.nframes_dev && order_frames(d->code.N, nframes, 2 * grid, max_iter)) {
+        if (own && !p.rows && !p.nframes_dev && orders(d, nframes, max_iter)) {
             void* order = (char*)d->msg + d->msg_cap;
             if (!cuda_ok(launch_order(llr, llr_stride, d->code.N, nframes, order, work + 1, d->sms, s), "frame order"))
                 return -1;
@@ -778,6 +787,13 @@ int drx_ldpc_decode_device(drx_ldpc* d, const int8_t* llr, size_t llr_stride, ui
     }
     return enqueue(d, llr, llr_stride, out, out_stride, iters, ok, nframes, max_iter, stop,
                    stream ? (cudaStream_t)stream : d->stream);
+}
+
+int drx_ldpc_decode_launches(const drx_ldpc* d, int nframes, int max_iter, int stop)
+{
+    if (!d || stop < 0)
+        return -1;
+    return nframes <= 0 ? 0 : stop == 0 && orders(d, nframes, max_iter) ? 2 : 1;
 }
 
 int drx_ldpc_set_learned(drx_ldpc* d, int iters, int nclass, const int8_t* class_of_degree,

@@ -100,6 +100,12 @@ int drx_ldpc_decode_device(drx_ldpc* d, const int8_t* llr, size_t llr_stride, ui
                            size_t out_stride, int32_t* iters, uint8_t* ok, int nframes,
                            int max_iter, int stop, void* stream);
 
+/* Kernels that drx_ldpc_decode_device launches for such a batch: the decoder,
+ * and before it, for larger batches of normal frames with per-frame stopping,
+ * the kernel that puts the frames in order (weakest first).  -1 for NULL or a
+ * stop below 0. */
+int drx_ldpc_decode_launches(const drx_ldpc* d, int nframes, int max_iter, int stop);
+
 /* No counterpart in the reference.  drx_ldpc_decode_device with per-frame
  * stopping for callers that must not allocate GPU memory on the decode path
  * (a real-time receiver thread, where cudaMalloc/cudaFree can stall on a
