@@ -9,14 +9,14 @@
  * GF(2^14) (short frames, x^14+x^5+x^3+x+1); W = deg g = 16 t or 14 t parity
  * bits; codewords of nbch = kldpc bits, MSB first, the highest degree first.
  *
- * k_bch_remainder: the remainders c(x) x^W mod g(x) of a batch, 8 or 32 lanes
+ * k_bch_remainder: the remainders c(x) x^W mod g(x) of a batch, 16 or 32 lanes
  * per frame; a zero remainder ends the frame (no error), the others are
  * queued.  The same kernel over the message bytes encodes.
- * k_bch_correct: one CTA per queued frame: syndromes, Berlekamp-Massey, the
- * roots of the locator over the whole field; when those at positions of the
- * shortened code number the degree, their bits are flipped.  For a
- * correctable word the locator is unique, so the result does not depend on
- * how it was found.
+ * k_bch_correct: up to four queued frames per CTA: syndromes and
+ * Berlekamp-Massey by a warp each, then the roots of one locator after the
+ * other over the whole field; when those at positions of the shortened code
+ * number the degree, their bits are flipped.  For a correctable word the locator
+ * is unique, so the result does not depend on how it was found.
  */
 #include <cuda_pipeline.h>
 #include <cuda_runtime.h>
@@ -78,8 +78,9 @@ struct BchBatch {
  * Bound by shared-memory reads: 18 reads of 256 bytes per step and warp, 36
  * of the 44 cycles that the load unit needs with the row loads; one thread per
  * frame over byte tables, as it was, waited for each step's reads in turn on
- * 64 threads' tables per CTA.  4096 normal 3/5 words without errors 0.260 ->
- * 0.037 ms; parity of 999 normal 9/10 words 0.532 -> 0.016 ms.  Half warps (n =
+ * 64 threads' tables per CTA.  A decode call of 4096 normal 3/5 words without
+ * errors 0.260 -> 0.061 ms, 0.042 of it this kernel; parity of 999 normal 9/10
+ * words 0.532 -> 0.016 ms.  Half warps (n =
  * 76 words) against whole warps (40) at 2048 words: 31 against 27 us, at 4096
  * no difference, so half a warp is taken once the batch has no warp for each.
  */
@@ -315,10 +316,12 @@ __host__ __device__ constexpr int triple_at(int i, int j, int k) { return k * (k
 
 constexpr int kMaxPts = 16 + 120 + 560;
 
-/* Carry-less product of two 16-bit values.  The factors are taken apart into
- * bits three apart, so that integer products add up without carries from one
- * result bit to the next: about 30 independent instructions, where a product
- * through logarithms waits for two loads from a table too large for L1. */
+/* Carry-less product of two 16-bit values, by masked integer products (the
+ * constant-time method of Pornin's BearSSL, "ctmul").  The factors are taken
+ * apart into bits four apart, so that the at most four terms of a result bit add
+ * up without a carry into the next bit of its class: about 30 independent
+ * instructions, where a product through logarithms waits for two loads from a
+ * table too large for L1. */
 __device__ __forceinline__ uint32_t clmul(uint32_t a, uint32_t b)
 {
     const uint32_t a0 = a & 0x1111u, a1 = a & 0x2222u, a2 = a & 0x4444u, a3 = a & 0x8888u;

@@ -310,11 +310,12 @@ __global__ void __launch_bounds__(256) k_demap(const __grid_constant__ DemapPara
 /* The same for rows that are all aligned and whole: symbols on 16 bytes, LLRs on
  * 8, symbol groups of four without a remainder, no padded label bits.  No row is
  * looked at for its alignment and no store for its end, and the pointers step:
- * 225 instructions for four 8PSK symbols, of which 186 are the distances,
- * minimums and roundings (287 in the general kernel).  4096 normal 8PSK frames
- * back to back 0.182 ms, 82 % of the measured HBM rate, which now binds; 0.241 in the general
- * kernel as it was, 0.227 with the minimums from a tree and the rounding by an
- * addition, 0.217 in this kernel with eight blocks per SM. */
+ * 245 warp instructions for four 8PSK symbols of 32 threads (counted over a
+ * launch).  4096 normal 8PSK frames take 0.194 to 0.205 ms a call, 72 to 76 % of
+ * the measured HBM rate, where the start of a call meets cold or dirty caches, and
+ * 0.180 (83 %) repeated without gaps, where HBM binds.  Without gaps it was 0.241
+ * in the general kernel as it was, 0.227 with the minimums from a tree and the
+ * rounding by an addition, 0.217 in this kernel with eight blocks per SM. */
 template <int BITS>
 __global__ void __launch_bounds__(256) k_demap_rows(const __grid_constant__ DemapParams p)
 {
@@ -394,7 +395,7 @@ cudaError_t launch_demap(const DemapParams& p, int sms, cudaStream_t s)
     const int gx = (((p.nsym + 3) / 4) + 255) / 256;
     /* 32 blocks per SM, of which five are resident (8PSK): a row of blocks takes a
      * few tens of frames, so the last ones leave no SM idle for long.  4096 normal
-     * frames at 8, 16, 32 and 64 blocks per SM: 8PSK 0.217, 0.191, 0.182, 0.179 ms,
+     * frames, repeated without gaps, at 8, 16, 32 and 64 blocks per SM: 8PSK 0.217, 0.191, 0.182, 0.179 ms,
      * QPSK 0.240, 0.216, 0.215, 0.209, 32APSK 0.317, 0.316, 0.319, 0.323; 512 8PSK
      * frames 28.0, 27.0, 27.1, 29.3 us.  (Five, one wave: 0.204 ms for 8PSK, 0.217
      * for QPSK.)  Two symbols' sums and products in one packed FP32 instruction gave

@@ -123,11 +123,11 @@ __device__ __forceinline__ uint32_t learned_lut(uint32_t c, uint32_t t)
  * which one changes no message), collected by a fused multiply-add per slot in
  * chains of about seven.
  *
- * Bound by the integer pipe and by issue: the decoder on 16-bit integers had 22
- * to 28 instructions of the integer pipe per link (minimums, selects, permutes
- * and both adds; the pipe 76 to 86 % busy with the other pipes idle), this form
- * about 13, its adds and selects on the other pipe.  us of the GPU per
- * frame-iteration before and after: S2X 18/30 0.305 and 0.206, normal 2/3 0.297
+ * Bound by issue: the decoder on 16-bit integers had 39 instructions of the
+ * integer pipe per link and frame pair of normal 3/5 (counted over a launch, level
+ * steps and syndrome included; the pipe 72 % busy, the FMA pipe 13 %), this form
+ * 25, its adds and selects on the FMA pipe (63 and 47 %).  us of the GPU per
+ * frame-iteration before and after this step alone: S2X 18/30 0.305 and 0.206, normal 2/3 0.297
  * and 0.279, 8/9 0.264 and 0.223, 9/10 0.331 and 0.257, short 1/2 0.086 and
  * 0.072, 3/5 0.143 and 0.117; normal 3/5 8PSK, 4096 frames over its waterfall
  * 37.4 and 31.3 ms.  Measured and not kept: link addresses two in a register or
@@ -579,7 +579,7 @@ __device__ int syndrome_pair(const DevCode& c, const PairFrame& fr, volatile int
  * 0.086, 3/5 0.181 -> 0.143, 5/6 0.182 -> 0.157 (all with the node on 16-bit
  * integers).  The forms are written out: one form over every slot's test that
  * takes the two smallest left normal 9/10 at 0.342 and 4/5 at 0.294, which run
- * at 0.257 and 0.249.
+ * at 0.250 and 0.261.
  */
 template <int KE, class Ck>
 __device__ __forceinline__ void read_late(Ck& ck, bool mine)

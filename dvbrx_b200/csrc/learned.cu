@@ -181,7 +181,7 @@ __device__ void load_params(const LearnedParams& p, int t, float* sbeta, float* 
  * level to level in shared memory.
  *
  * Bound by the dependent steps of a frame's layers: one frame alone on an SM
- * takes 0.65 ms per iteration forward and backward, three or four 1.6 ms; DRAM
+ * takes 0.65 ms per iteration forward and backward, three or four 1.7 ms; DRAM
  * is under 20 %.  512 normal 2/3 frames, 20 iterations, loss and gradients:
  * 73.5 ms with the whole check node in every level step, 33.7 ms so.  (Extrinsic
  * inputs and message gradients fetched a layer ahead into shared memory: 34.6;

@@ -150,7 +150,7 @@ int drx_channel_generate(drx_ldpc* d, const char* constellation, const char* con
                          void* stream);
 
 /* Kernel of the per-frame batch calls: DRX_VARIANT_AUTO (the default) runs
- * the frame-pair kernel (two frames per CTA, 16x2 SIMD), which covers every
+ * the frame-pair kernel (two frames per CTA, FP16 pairs), which covers every
  * code; DRX_VARIANT_FRAME pins the one-frame kernel.  Both give identical
  * results.  Returns the
  * variant per-frame batches will now run (DRX_VARIANT_FRAME or
